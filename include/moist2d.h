@@ -481,7 +481,8 @@ int moist_step_profile(moist_ctx* ctx, int nsteps, float* total_ms, float* group
                        long long* group_launches);
 
 /* Diagnostic of the tiled tracer sweep: counts[p] (p < n, p < 64) = sweeps since the last call
- * that reached their bitwise fixed point after p passes; the counters are reset.
+ * that reached their bitwise fixed point after p passes (of all chunks; 63: or more); the counters are
+ * reset.
  * MOIST_ERR_UNSUPPORTED when the context runs the wavefront sweep. */
 int moist_tracer_pass_counts(moist_ctx* ctx, int* counts, int n);
 
@@ -499,7 +500,9 @@ int moist_set_wait_limit(moist_ctx* ctx, long long cycles);
  * steps (3 sweeps each) with every pass timed on the device. For sweep w (0 .. 3*nsteps-1):
  * npasses[w] = passes run; pass_ns[w*maxrec + q] = duration of pass q+1 in ns (from its start to
  * the next pass's start, the last one to the moment block 0 leaves the sweep);
- * pass_tiles[w*maxrec + q] = tile-tracer warps that recomputed in that pass (3 per tile at most).
+ * pass_tiles[w*maxrec + q] = work of that pass: tile-tracer warps (16 rows x 32 columns each) that
+ * recomputed, two counted as one (rounded up), so 3 per 32 x 32 cells at most. A domain whose tiles do
+ * not all fit on the GPU is swept in chunks of tile columns: the passes traced are the first chunk's.
  * In the dataflow form a "pass" is a tile's q-th computation: npasses is the largest count of
  * any tile, pass_tiles counts the tile-tracer warps that computed a q-th time, and pass_ns is the
  * difference between the latest starts of computations q+1 and q+2 (or the end). Any output

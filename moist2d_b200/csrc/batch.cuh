@@ -101,9 +101,7 @@ struct BSub {
 template <class T>
 struct BPrep {
     DevParams<T> p;
-    TracerArgs<T> tr;
-    T *s0, *s1, *s2;
-    double* rrho;
+    StreamArgs<T> a;
     const int* err;
 };
 template <class T>
@@ -210,7 +208,7 @@ constexpr int BATCH_COL_THREADS = 64;
 template <class T>
 struct FPrep {
     __device__ void operator()(const BPrep<T>& a, int bx, int by) const {
-        b_stream_prep(a.p, a.tr, a.s0, a.s1, a.s2, a.rrho, a.err, bx, by);
+        b_stream_prep(a.p, a.a, a.err, bx, by);
     }
 };
 template <class T>

@@ -13,6 +13,8 @@
 
 #include <cuda_runtime.h>
 
+#include "moist_math.h"
+
 namespace moist {
 
 // The sign of a zero result: for a nonzero quotient q and q0 (two roundings of the same value)
@@ -35,12 +37,18 @@ __device__ __forceinline__ float sel_lt(float a, float b, float x, float y) {  /
         : "=f"(r) : "f"(a), "f"(b), "f"(x), "f"(y));
     return r;
 }
+__device__ __forceinline__ double sel_gt(double a, double b, double x, double y) { return a > b ? x : y; }
+__device__ __forceinline__ double sel_lt(double a, double b, double x, double y) { return a < b ? x : y; }
+__device__ __forceinline__ double sel_u(unsigned c, double x, double y) { return c != 0 ? x : y; }
 __device__ __forceinline__ float sel_u(unsigned c, float x, float y) {  // c != 0 ? x : y
     float r;
     asm("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %1, 0;\n\tselp.f32 %0, %2, %3, p;\n\t}"
         : "=f"(r) : "r"(c), "f"(x), "f"(y));
     return r;
 }
+
+__device__ __forceinline__ bool same_bits(float x, float y) { return __float_as_uint(x) == __float_as_uint(y); }
+__device__ __forceinline__ bool same_bits(double x, double y) { return __double_as_longlong(x) == __double_as_longlong(y); }
 
 // Julia's min / max (NaN-propagating, -0 < +0) as single PTX instructions
 __device__ __forceinline__ float jmin_f(float a, float b) {
@@ -53,6 +61,8 @@ __device__ __forceinline__ float jmax_f(float a, float b) {
     asm("max.NaN.f32 %0, %1, %2;" : "=f"(r) : "f"(a), "f"(b));
     return r;
 }
+__device__ __forceinline__ double jmin_f(double a, double b) { return mm::jmin(a, b); }
+__device__ __forceinline__ double jmax_f(double a, double b) { return mm::jmax(a, b); }
 
 // ---- FP64-reciprocal division: RN32(a/b) = RN32(RN64(a * y)) for y = 1/b to within 2^-51
 //
@@ -129,6 +139,142 @@ struct Div64X {  // FP64 reciprocal with explicit rounding of subnormal quotient
     __device__ __forceinline__ static float div3(float a) { return div64(a, 1.0 / 3.0); }
 };
 
+// ---- division in the type's own arithmetic: remainder corrections on a reciprocal
+//
+// Let q0 be within one ulp of a/b. Its remainder a - b q0 is then a float (the FMA forms it
+// exactly), and RN(q0 + (a - b q0) RN(1/b)) = RN(a/b) (P. Markstein, IBM J. Res. Dev. 34, 1990;
+// the quotient theorem of Muller et al., Handbook of Floating-Point Arithmetic). The remainder
+// must not underflow: it is formed from the numerator and q0 scaled by UP (both exact), and the
+// last FMA takes it back with RN(1/b) / UP onto the unscaled q0, so a subnormal quotient too is
+// rounded once, onto its own grid. There the argument holds but for exact ties (the rounding
+// error of 1/b decides them): a tie is |remainder| = b times half a grid unit. cdiv sends it to the
+// even neighbour (the tails at the edges of clouds fall through the subnormal range within a few
+// cells, where every hundredth or so quotient by 100 or 250 is one); in quot and ratio, whose
+// denominators have long significands, it sets `bad`.
+//   prepared b (cdiv): q0 = RN(a d + RN(a l)) with d + l = 1/b to 2^-40, and one correction;
+//   variable b: RN(1/b) from the hardware approximation, q0 = RN(a RN(1/b)) is within 1.5 ulp,
+//   one correction makes it one of the two values around a/b, a second one RN(a/b).
+// d is 1/b rounded down, so that both terms of q0 and the correction of a zero keep the sign of a
+// zero numerator (b > 0). What leaves the admitted ranges ends as a non-finite result or sets
+// `bad`, never as a wrong finite one: a prepared denominator outside [LO, HI] has NaN
+// reciprocals, |a| UP and q0 UP overflow to infinities that the correction turns into an
+// infinity or NaN, a variable denominator above BIG sets `bad`. The sweeps check `bad` and the
+// finiteness of their results once per tile or sweep and repeat it with IeeeDiv.
+// tests/celldiv_check.cu compares every primitive with IEEE division on the GPU: all 2^32 numerators for
+// the model's denominators, all 2^32 denominators for the reciprocal, and random bit patterns.
+//
+// Against a multiplication by the reciprocal in double precision (Div64) this leaves out the two
+// conversions of every quotient, which an SM issues at 16 lanes a cycle (a quarter of a warp's
+// FMA rate per scheduler); against CUDA's division it has no branch.
+template <class T>
+struct Rcp {        // reciprocal of a prepared denominator b
+    T d, l, n;      // 1/b rounded down, the rest 1/b - d, and RN(1/b) / UP
+    T tie;          // the remainder of an exact subnormal tie (-1 for a power of two)
+};
+
+template <class T>
+struct DivRange;
+template <>
+struct DivRange<float> {
+    static constexpr float UP = 0x1p64f, DOWN = 0x1p-64f, TIE = 0x1p-86f;  // TIE = 2^-150 UP
+    static constexpr float LO = 0x1p-40f, HI = 0x1p40f, BIG = 0x1p60f, MAX = 0x1.fffffep127f;
+};
+template <>
+struct DivRange<double> {
+    static constexpr double UP = 0x1p200, DOWN = 0x1p-200, TIE = 0x1p-875;  // TIE = 2^-1075 UP
+    static constexpr double LO = 0x1p-100, HI = 0x1p100, BIG = 0x1p800, MAX = 0x1.fffffffffffffp1023;
+};
+
+__device__ __forceinline__ float fma_t(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ bool odd(float x) { return (__float_as_uint(x) & 1u) != 0u; }
+__device__ __forceinline__ bool odd(double x) { return (__double_as_longlong(x) & 1ll) != 0; }
+__device__ __forceinline__ double fma_t(double a, double b, double c) { return __fma_rn(a, b, c); }
+
+__device__ __forceinline__ float rcp_rd(float b) { return __frcp_rd(b); }
+__device__ __forceinline__ double rcp_rd(double b) { return __drcp_rd(b); }
+
+// RN(1/b) of a variable denominator: the hardware approximation and Newton steps. Float: one
+// step, checked against IEEE division for every |b| in [2^-125, 2^125]. Double: two steps reach
+// one ulp, the third gives RN(1/b) unless b's significand is all ones (Markstein), which sets bad.
+__device__ __forceinline__ float rcp_rn(float b, bool&) {
+    float y;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
+    return __fmaf_rn(y, __fmaf_rn(-b, y, 1.0f), y);
+}
+__device__ __forceinline__ double rcp_rn(double b, bool& bad) {
+    double y;
+    asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
+    y = __fma_rn(y, __fma_rn(-b, y, 1.0), y);
+    y = __fma_rn(y, __fma_rn(-b, y, 1.0), y);
+    bad |= ((unsigned long long)__double_as_longlong(b) << 12) == 0xfffffffffffff000ull;
+    return __fma_rn(y, __fma_rn(-b, y, 1.0), y);
+}
+
+template <class T>
+struct FastDiv : DivRange<T> {
+    using DR = DivRange<T>;
+    __device__ __forceinline__ static Rcp<T> prep(T b) {
+        if (!(b >= DR::LO && b <= DR::HI)) {
+            const T nan = T(0) / T(0);
+            return {nan, nan, nan, nan};
+        }
+        const T y = T(1) / b, d = rcp_rd(b), e = fma_t(-b, d, T(1));  // 1 - b d is exact
+        return {d, e * y, y * DR::DOWN, e == T(0) ? T(-1) : b * DR::TIE};
+    }
+    // RN(1/b) of a prepared denominator for quot()
+    __device__ __forceinline__ static T prep1(T b) { return b >= DR::LO && b <= DR::HI ? T(1) / b : T(0) / T(0); }
+    __device__ __forceinline__ static T cdiv(T a, T b, const Rcp<T>& y) {
+        const T q0 = fma_t(a, y.d, a * y.l);
+        const T rn = fma_t(b, q0 * DR::UP, -(a * DR::UP));  // negated: +0 for a zero of either sign
+        // on a tie the correction with a slightly larger reciprocal reaches the other neighbour
+        const T other = fma_t(-rn, y.n * T(1.0000305), q0);
+        return fabs(rn) == y.tie ? (odd(q0) ? other : q0) : fma_t(-rn, y.n, q0);
+    }
+    __device__ __forceinline__ static T twice(T a, T b, T y, T tie, bool& bad) {
+        const T as = -(a * DR::UP), n = y * DR::DOWN;
+        T q = a * y;
+        q = fma_t(-fma_t(b, q * DR::UP, as), n, q);
+        const T rn = fma_t(b, q * DR::UP, as);
+        bad |= fabs(rn) == tie;
+        return fma_t(-rn, n, q);
+    }
+    // a / b with y = prep1(b)
+    __device__ __forceinline__ static T quot(T a, T b, T y, bool& bad) { return twice(a, b, y, b * DR::TIE, bad); }
+    // the limiter ratio: |b| < EPS ? 1 : a / b (the sign of a zero is not kept for b < 0: the limiter
+    // takes both zeros to +0)
+    __device__ __forceinline__ static T ratio(T a, T b, T EPS, bool& bad) {
+        const T ab = fabs(b);
+        const bool one = ab < EPS;
+        bool refuse = ab > DR::BIG;
+        const T y = rcp_rn(b, refuse);
+        const T q = twice(a, b, y, ab * DR::TIE, refuse);
+        bad |= !one && refuse;
+        return one ? T(1) : q;
+    }
+    // (1 + 2 r) / 3: the numerator is 0 or at least 2^-24 (2^-53) in magnitude. Float: 1/3 as two
+    // floats and one FMA, checked for every numerator of 2^-30 to 2^120.
+    __device__ __forceinline__ static T div3(T a) {
+        if constexpr (sizeof(T) == 4) {
+            constexpr float yh = 1.0f / 3.0f, yl = (float)(1.0 / 3.0 - (double)yh);
+            return __fmaf_rn(a, yh, a * yl);
+        } else {
+            constexpr double y = 1.0 / 3.0;
+            double q = a * y;
+            q = __fma_rn(__fma_rn(-3.0, q, a), y, q);
+            return __fma_rn(__fma_rn(-3.0, q, a), y, q);
+        }
+    }
+};
+
+// the same interface with IEEE division
+template <class T>
+struct IeeeDiv {
+    __device__ __forceinline__ static T cdiv(T a, T b, const Rcp<T>&) { return a / b; }
+    __device__ __forceinline__ static T quot(T a, T b, T, bool&) { return a / b; }
+    __device__ __forceinline__ static T ratio(T a, T b, T EPS, bool&) { return fabs(b) < EPS ? T(1) : a / b; }
+    __device__ __forceinline__ static T div3(T a) { return a / T(3); }
+};
+
 // ---- the correctly rounded double quotient a/b without a division on the dependent path
 //
 // Given y = RN(1/b) (formed ahead, off the path): q0 = RN(a y) lies within 1.5 ulp of a/b; one
@@ -161,14 +307,5 @@ __device__ __forceinline__ double qdiv_checked(double a, double b, double y, boo
     ok = ok && (zero || (in_range && fabs(r1) < ab * half_u));
     return zero ? q0 : q1;
 }
-
-// division policies for the templated tracer arithmetic: div(a, b) with a variable
-// denominator, divr(a, b, y) with y = RN(1/b) prepared in advance
-template <class T>
-struct DivIEEE {
-    __device__ __forceinline__ static T div(T a, T b, bool&) { return a / b; }
-    __device__ __forceinline__ static T divr(T a, T b, T, bool&) { return a / b; }
-};
-
 
 }  // namespace moist

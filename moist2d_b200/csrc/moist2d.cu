@@ -233,6 +233,7 @@ struct Ctx : CtxBase {
     // tiled tracer sweep (tracer_tiles.cuh)
     bool use_tiles = false;
     bool tiles_df = false;  // the tiled sweep without grid barriers (per-tile versions)
+    bool tiles_df_fit = false;  // it needs every tile resident
     TileCtl tctl{};
     T* strips = nullptr;
     int* pass_hist = nullptr;  // [64] sweeps that converged after p passes
@@ -241,8 +242,7 @@ struct Ctx : CtxBase {
     StepRecord* rec = nullptr;
     // row-streaming tracer sweep (MOIST_FLAG_TRACER_STREAM)
     bool use_stream = false;
-    T* s_old[3] = {nullptr, nullptr, nullptr};
-    double* rrho = nullptr;
+    T *skew_dom = nullptr, *skew_trc[3] = {nullptr, nullptr, nullptr};  // its records by anti-diagonal
     // column strips of the factorisation and the acoustic substeps
     int strip_wc = 1;
     size_t strip_smem = 0;
@@ -418,13 +418,24 @@ struct Ctx : CtxBase {
             if (nz > STREAM_MAX_ROWS)
                 return set_err(owner, MOIST_ERR_UNSUPPORTED, "the streaming tracer sweep needs nz <= %d (got %d)",
                                STREAM_MAX_ROWS, nz);
-            for (int t = 0; t < 3; t++) AL(s_old[t], fsz);
-            AL(rrho, fsz);
+            if (int r = alloc_stream()) return r;
             use_stream = true;
         }
         if (int r = init_tiles()) return r;
         CK(reset_err());
         CK(cudaStreamSynchronize(st));
+        return MOIST_OK;
+    }
+
+    // the records of the streaming sweep (zero where no cell writes them)
+    int alloc_stream() {
+        const size_t n = skew_rows(nx, nz) * skew_pitch(nz);
+        AL(skew_dom, n * SK_ND);
+        for (int t = 0; t < 3; t++) AL(skew_trc[t], n * SK_NT);
+        int dev = 0, optin = 0;
+        CK(cudaGetDevice(&dev));
+        CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
+        CK(cudaFuncSetAttribute(k_tracer_stream<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
         return MOIST_OK;
     }
 
@@ -457,13 +468,13 @@ struct Ctx : CtxBase {
         return MOIST_OK;
     }
 
-    // The tiled sweep needs every tile resident at once (its passes meet at grid barriers);
-    // otherwise, or when MOIST_FLAG_TRACER_WAVEFRONT is set, the exact wavefront runs instead.
+    // The tiled sweep needs the tiles of a chunk (all rows of a number of tile columns) resident at once
+    // (its passes meet at grid barriers): as many columns as fit, in chunks of about equal width.
+    // When MOIST_FLAG_TRACER_WAVEFRONT is set, the exact wavefront runs instead.
     int init_tiles() {
         tctl.tiles_x = (nx + TT_W - 1) / TT_W;
-        tctl.tiles_z = (nz + TT_W - 1) / TT_W;
+        tctl.tiles_z = (nz + TT_H - 1) / TT_H;
         tctl.ntiles = tctl.tiles_x * tctl.tiles_z;
-        tctl.max_pass = tctl.tiles_x + tctl.tiles_z + 2;
         tile_smem = sizeof(TileSmem<T>);
         if (owner->flags & (MOIST_FLAG_TRACER_WAVEFRONT | MOIST_FLAG_TRACER_STREAM)) return MOIST_OK;
         int dev = 0, nsm = 0, coop = 0, nb = 0;
@@ -471,16 +482,23 @@ struct Ctx : CtxBase {
         CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
         CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
         CK(cudaFuncSetAttribute(k_tracer_tiles<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_smem));
+        CK(cudaFuncSetAttribute(k_tracer_tiles<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_smem));
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_tracer_tiles<T, false>, 96, tile_smem));
-        if (!coop || (long)nb * nsm < tctl.ntiles) return MOIST_OK;
-        // the barrier sweep uses two parities of strips, the dataflow sweep TT_RING versions
-        AL(strips, (size_t)std::max(2, TT_RING) * 3 * tctl.ntiles * 4 * TT_W);
+        const int fit = nb * nsm / tctl.tiles_z;  // tile columns
+        if (!coop || fit < 1) return MOIST_OK;
+        const int nchunk = (tctl.tiles_x + fit - 1) / fit;
+        tctl.chunk_x = (tctl.tiles_x + nchunk - 1) / nchunk;
+        tctl.max_pass = tctl.chunk_x + tctl.tiles_z + 2;
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_tracer_tiles<T, true>, 96, tile_smem));
+        tiles_df_fit = nchunk == 1 && nb * nsm >= tctl.ntiles;
+        // the dataflow sweep uses TT_RING versions of the strips
+        AL(strips, (size_t)TT_RING * 3 * tctl.ntiles * 4 * TT_W);
         AL(tctl.ver, (size_t)3 * tctl.ntiles);
-        AL(tctl.bar, 2);
+        AL(tctl.bar, 3);
         AL(tctl.changed, (size_t)2 * 3 * tctl.ntiles * 2);
-        AL(tctl.any_changed, (size_t)tctl.max_pass + 2);
         AL(tctl.passes, 1);
         AL(pass_hist, 64);
+        tctl.hist = pass_hist;
         tctl.pass_ts = nullptr;
         tctl.pass_work = nullptr;
         tctl.timeout = err + 2;
@@ -489,8 +507,7 @@ struct Ctx : CtxBase {
         tctl.spin_limit = (long long)clk * 1000LL * 2;                 // about two seconds
         wait_default = tctl.spin_limit;
         use_tiles = true;
-        tiles_df = (owner->flags & MOIST_FLAG_TRACER_DATAFLOW) != 0;
-        CK(cudaFuncSetAttribute(k_tracer_tiles<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_smem));
+        tiles_df = tiles_df_fit && (owner->flags & MOIST_FLAG_TRACER_DATAFLOW) != 0;
         return MOIST_OK;
     }
 
@@ -503,7 +520,7 @@ struct Ctx : CtxBase {
         if (h[2] != 0) {
             // the blocks that gave up left the barrier words mid-count: clear them and the flag
             // so that the context can step again (from a State uploaded anew)
-            if (tctl.bar) CK(cudaMemsetAsync(tctl.bar, 0, 2 * sizeof(unsigned), st));
+            if (tctl.bar) CK(cudaMemsetAsync(tctl.bar, 0, 3 * sizeof(*tctl.bar), st));
             CK(reset_err());
             CK(cudaStreamSynchronize(st));
             return set_err(owner, MOIST_ERR_TIMEOUT, "a grid barrier of the tiled tracer sweep timed out");
@@ -835,20 +852,19 @@ struct Ctx : CtxBase {
         tr.dt = dt_stage;
         MARK(MOIST_KGROUP_TRACER, (use_stream || use_tiles) ? 2 : 1);
         if (use_stream) {
-            StreamArgs<T> sa{tr, {s_old[0], s_old[1], s_old[2]}, rrho};
+            StreamArgs<T> sa{tr, skew_dom, {skew_trc[0], skew_trc[1], skew_trc[2]}};
             if (rec) {
-                rec->put(BK_PREP, BPrep<T>{dp, tr, s_old[0], s_old[1], s_old[2], rrho, err});
+                rec->put(BK_PREP, BPrep<T>{dp, sa, err});
                 rec->put(BK_STREAM, BStream<T>{dp, sa, err});
             } else {
-                k_stream_prep<T><<<g2, b2, 0, st>>>(dp, tr, s_old[0], s_old[1], s_old[2], rrho, err);
+                k_stream_prep<T><<<dim3(cdiv(nx + 3, 32), cdiv(nz, 32)), 256, 0, st>>>(dp, sa, err);
                 CKL();
-                k_tracer_stream<T><<<3, (nz + 31) / 32 * 32, 0, st>>>(dp, sa, err);
+                k_tracer_stream<T><<<3, stream_threads(nz), stream_smem_bytes<T>(nz), st>>>(dp, sa, err);
                 CKL();
             }
         } else if (rec) {
             return set_err(owner, MOIST_ERR_UNSUPPORTED, "a recorded step needs the streaming tracer sweep");
         } else if (use_tiles) {
-            CK(cudaMemsetAsync(tctl.any_changed, 0, (tctl.max_pass + 2) * sizeof(int), st));
             TileCtl c = tctl;
             if (trace_ts && trace_n < trace_cap) {  // moist_tracer_pass_trace
                 const size_t stride = (size_t)tctl.max_pass + 3;
@@ -864,12 +880,12 @@ struct Ctx : CtxBase {
                 CK(cudaMemsetAsync(tctl.passes, 0, sizeof(int), st));
                 CK(cudaLaunchCooperativeKernel((void*)k_tracer_tiles<T, true>, dim3(tctl.ntiles), dim3(96), args,
                                                tile_smem, st));
+                k_pass_count<<<1, 1, 0, st>>>(tctl.passes, pass_hist);
+                CKL();
             } else {
-                CK(cudaLaunchCooperativeKernel((void*)k_tracer_tiles<T, false>, dim3(tctl.ntiles), dim3(96), args,
-                                               tile_smem, st));
+                CK(cudaLaunchCooperativeKernel((void*)k_tracer_tiles<T, false>, dim3(tctl.chunk_x * tctl.tiles_z),
+                                               dim3(96), args, tile_smem, st));
             }
-            k_pass_count<<<1, 1, 0, st>>>(tctl.passes, pass_hist);
-            CKL();
         } else {
             const int nthr = (nz + 31) / 32 * 32;
             k_tracer_wavefront<T><<<3, nthr, 3 * nz * sizeof(T), st>>>(dp, tr, err);
@@ -1037,7 +1053,7 @@ struct Ctx : CtxBase {
                     d = (long long)(t1 - t[q + 1]);
                 }
                 if (pass_ns) pass_ns[w * maxrec + q] = d;
-                if (pass_tiles) pass_tiles[w * maxrec + q] = (q + 1 <= np) ? k[q + 1] : 0;
+                if (pass_tiles) pass_tiles[w * maxrec + q] = (q + 1 <= np) ? (k[q + 1] + 1) / 2 : 0;  // warps of 16 rows, in tiles of 32
             }
         }
         return finish();
@@ -1219,10 +1235,8 @@ struct Ctx : CtxBase {
         int dev = 0, optin = 0;
         CK(cudaGetDevice(&dev));
         CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-        if (nz <= STREAM_MAX_ROWS && !s_old[0]) {  // buffers of the streaming sweep
-            for (int t = 0; t < 3; t++) AL(s_old[t], fsz);
-            AL(rrho, fsz);
-        }
+        if (nz <= STREAM_MAX_ROWS && !skew_dom)
+            if (int r = alloc_stream()) return r;
         std::array<T*, 8>& save = tune_save;
         if (!save[0]) {  // kept for later calls
             for (int f = 0; f < 7; f++) AL(save[f], fsz);
@@ -1250,8 +1264,9 @@ struct Ctx : CtxBase {
         };
         std::vector<Cand> cands;
         for (int tr = 0; tr < 3; tr++) {
-            if (tr != 1 && !strips) continue;  // the tiles need all of them resident (init_tiles)
-            if (tr == 1 && !s_old[0]) continue;
+            if (tr != 1 && !strips) continue;  // the context has no tiles (init_tiles)
+            if (tr == 2 && !tiles_df_fit) continue;
+            if (tr == 1 && !skew_dom) continue;
             for (int w : {1, 2, 4, 8})
                 if (w <= nx && strip_smem_bytes<T, TT>(nz, w) <= (size_t)optin) cands.push_back({w, tr});
         }
@@ -1952,8 +1967,8 @@ struct BatchImpl : BatchBase {
     std::vector<void*> allocs;
     int col_threads = BATCH_COL_THREADS;  // threads per block of the per-column kernels
     bool sub_strips = false;               // factorisation and substep over column strips instead
-    int stream_minb = 1;                   // register bound of the streaming tracer sweep: 1 or 2 blocks of
-                                           // 256 threads per SM, or 3 blocks of 128 (rows <= 128)
+    int stream_minb = 2;                   // register bound of the streaming tracer sweep: 2 or 3 blocks of
+                                           // 256 threads per SM (rows <= 128), 1: one block of 512
     // per-column substep body: 0 b_substep_col (64 registers), 1 and 2 b_substep_col_pf (loads one
     // level ahead; 128 and 85 registers), 3 and 4 b_substep_col_async (the next level copied into
     // shared memory; 85 and 128 registers), 5 the same two levels ahead (128 registers)
@@ -2018,10 +2033,16 @@ struct BatchImpl : BatchBase {
             case BK_DIAG:
             case BK_TEND:
             case BK_UPD:
-            case BK_PREP:
                 block = dim3(32, 8);
                 for (int i = 0; i < n; i++)
                     if (in_group(i)) cells(i);
+                break;
+            case BK_PREP:
+                block = dim3(256);
+                for (int i = 0; i < n; i++)
+                    if (in_group(i))
+                        for (unsigned by = 0; by < cdiv(m[i]->nz, 32); by++)
+                            for (unsigned bx = 0; bx < cdiv(m[i]->nx + 3, 32); bx++) it.push_back({i, (int)bx, (int)by});
                 break;
             case BK_THOMAS:
             case BK_SUB:
@@ -2042,7 +2063,12 @@ struct BatchImpl : BatchBase {
                 break;
             case BK_STREAM: {
                 // the longest sweeps (nx + nz steps) first, so that the short ones fill the tail
-                block = dim3(max_rows);
+                block = dim3(32);
+                for (int i = 0; i < n; i++)
+                    if (in_group(i)) {
+                        block.x = std::max<unsigned>(block.x, stream_threads(m[i]->nz));
+                        smem = std::max(smem, stream_smem_bytes<T>(m[i]->nz));
+                    }
                 std::vector<int> order(n);
                 for (int i = 0; i < n; i++) order[i] = i;
                 order.erase(std::remove_if(order.begin(), order.end(), [&](int i) { return !in_group(i); }), order.end());
@@ -2162,14 +2188,14 @@ struct BatchImpl : BatchBase {
                 break;
             BATCH_LAUNCH(BK_PREP, BPrep<T>, FPrep<T>, 4)
             case BK_STREAM:
-                if (stream_minb == 2)  // registers bounded so that twice the blocks fit on an SM
-                    k_batched<BStream<T>, FStream<T>, 2><<<s.nitems, s.block, s.smem, ls>>>(
+                if (s.block.x > 256 || stream_minb == 1)
+                    k_batched_b<BStream<T>, FStream<T>, 2 * STREAM_MAX_ROWS, 1><<<s.nitems, s.block, s.smem, ls>>>(
                         s.items, (const BStream<T>*)s.args, FStream<T>{});
-                else if (stream_minb == 3)  // blocks of at most 128 threads, three of them per SM
-                    k_batched_b<BStream<T>, FStream<T>, 128, 3><<<s.nitems, s.block, s.smem, ls>>>(
+                else if (stream_minb == 2)  // registers bounded so that two blocks of 256 threads fit on an SM
+                    k_batched_b<BStream<T>, FStream<T>, 256, 2><<<s.nitems, s.block, s.smem, ls>>>(
                         s.items, (const BStream<T>*)s.args, FStream<T>{});
-                else
-                    k_batched<BStream<T>, FStream<T>, 1><<<s.nitems, s.block, s.smem, ls>>>(
+                else  // or three
+                    k_batched_b<BStream<T>, FStream<T>, 256, 3><<<s.nitems, s.block, s.smem, ls>>>(
                         s.items, (const BStream<T>*)s.args, FStream<T>{});
                 break;
             BATCH_LAUNCH(BK_UPD, BUpd<T>, FUpd<T>, 4)
@@ -2528,6 +2554,12 @@ struct BatchImpl : BatchBase {
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
             BCK(cudaFuncSetAttribute(k_batched<SINGLE_ARG(BSub<T, TT>), SINGLE_ARG(FSubAsync<T, TT, 3>), 2>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
+            BCK(cudaFuncSetAttribute(k_batched_b<BStream<T>, FStream<T>, 2 * STREAM_MAX_ROWS, 1>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
+            BCK(cudaFuncSetAttribute(k_batched_b<BStream<T>, FStream<T>, 256, 2>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
+            BCK(cudaFuncSetAttribute(k_batched_b<BStream<T>, FStream<T>, 256, 3>,
+                                     cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
             BCK(cudaFuncSetAttribute(k_batched_b<ASolve, FASubSolve, ADJ_SOLVE_THREADS, 1>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
         }
@@ -2747,7 +2779,7 @@ struct BatchImpl : BatchBase {
         int bmb = stream_minb;
         float best_mb = 1e30f;
         for (int mb : {1, 2, 3}) {
-            if (mb == 3 && max_rows > 128) continue;  // the 128-thread bound needs rows <= 128
+            if (mb > 1 && max_rows > 128) continue;  // the 256-thread bounds need rows <= 128
             stream_minb = mb;
             if (int r = set_col_threads(bct)) return r;  // recaptures the graphs
             if (int r = copy_all(false)) return r;

@@ -1,37 +1,43 @@
 // tracer_stream.cuh - the reference's in-place Gauss-Seidel tracer sweep as one exact wavefront
-// per tracer, streaming every row through registers.
+// per tracer, streaming the anti-diagonals of the domain through shared memory.
 //
 // Cell (k, i) of the in-place sweep (moist.jl:1469-1518) reads the updated values at (k, i-1),
 // (k, i-2), (k-1, i), (k-2, i) and stage-start values elsewhere, so the anti-diagonals
-// k + i = const can be updated together. One block sweeps one tracer of one domain: thread k
-// owns row k (nz <= STREAM_MAX_ROWS) and updates column c = s - k at step s, for
-// s = 0 .. nx + nz - 2. No speculation, no repair passes and no grid-wide barrier: blocks are
-// independent, so any number of (domain, tracer) sweeps can share one launch.
+// k + i = const can be updated together. One block sweeps one tracer of one domain: two lanes own
+// row k (tracer_cell.cuh; 16 rows per warp, nz <= STREAM_MAX_ROWS) and update column c = s - k at
+// step s, for s = 0 .. nx + nz - 2. No speculation, no repair passes and no grid-wide barrier:
+// blocks are independent, so any number of (domain, tracer) sweeps can share one launch.
 //
-// Each thread keeps a window of its own row (stage-start s = rho_q / rho at c .. c+2, density
-// at c-1 .. c+1, mfx at c-1, c, mfz at c-1, c) and loads the next column one step ahead. The
-// neighbouring rows come from the neighbouring threads, which stand one column behind (row
-// k+1) or ahead (row k-1): warp shuffles inside a warp; across a warp boundary the stage-start
-// values are loaded directly and the two updated values of the top rows of the warp below go
-// through a small shared-memory ring, one block barrier per step.
-//
-// The cell update is the Float32 branch-free cell of tracer_tiles.cuh (FP64-reciprocal
-// division, exact fallback) or the IEEE cell for Float64: the same operations as the tiled
-// sweep, so the two kernels agree bit for bit.
+// The stage-start inputs are first copied by b_stream_prep into records by anti-diagonal (element
+// k of record s belongs to column s - k), so that a step reads whole lines: with the fields' own
+// layout every lane of a load touches another row, 32 lines a load, which bounded the sweep (2900
+// cycles a step with two or three blocks of 128 rows on an SM). The block copies one record a step with
+// 16-byte cp.async into a ring of shared memory, three steps before its first use. The updated
+// values of the rows below come through warp shuffles, across warps through a small ring, one
+// block barrier per step.
 #pragma once
 
 #include "tracer_tiles.cuh"
 
 namespace moist {
 
-constexpr int STREAM_MAX_ROWS = 256;  // rows per block (threads); the register budget allows no more
-constexpr int STREAM_RING = 8;        // columns kept of the two top rows of every warp
+constexpr int STREAM_MAX_ROWS = 256;  // rows per block (two threads each)
+constexpr int STREAM_RING = 8;        // records in shared memory; columns kept of the two top rows of every warp
+
+// fields of a record: the first six are the domain's, the last three the tracer's
+enum { SK_VX = 0, SK_VZ, SK_RX, SK_RZ, SK_RHO, SK_RRHO, SK_ND, SK_S = 0, SK_Q0, SK_DPH, SK_NT };
+
+// elements of one field of a record: rows -1 .. nz+1 at positions 0 .. nz+2, padded to 16 (mod 32) so that
+// the two halves of a warp read two neighbouring fields on different banks
+__host__ __device__ inline int skew_pitch(int nz) { return (nz + 3 + 15) / 32 * 32 + 16; }
+// records s = -1 .. nx + nz + 1 (+ the ring's look-ahead)
+__host__ __device__ inline size_t skew_rows(int nx, int nz) { return (size_t)nx + nz + 4 + STREAM_RING; }
 
 template <class T>
 struct StreamArgs {
     TracerArgs<T> tr;
-    const T* s_old[3];   // stage-start rho_q / rho, [nz][P]
-    const double* rrho;  // 1 / rho in double precision, [nz][P] (Float32 fast cell)
+    T* dom;      // [skew_rows][SK_ND][pitch]
+    T* trc[3];   // [skew_rows][SK_NT][pitch]
 };
 
 __device__ __forceinline__ int pmod(int c, int n) {
@@ -39,253 +45,193 @@ __device__ __forceinline__ int pmod(int c, int n) {
     return r < 0 ? r + n : r;
 }
 
-// stage-start s = rho_q / rho and the reciprocal densities of the stream sweep
+// The records of the sweep: block (bx, by) takes columns 32 bx - 1 .. 32 bx + 30 of rows 32 by ..
+// 32 by + 31 (256 threads), reads every field by rows and writes it by anti-diagonals through a
+// shared tile. s = rho_q / rho (IEEE), the reciprocal of rho for quot(), face densities. Positions no
+// cell of the domain has (rows -1, nz, nz+1; corners) keep the zeros of the allocation.
 template <class T>
-__device__ __forceinline__ void b_stream_prep(DevParams<T> p, TracerArgs<T> a, T* s0, T* s1, T* s2, double* rrho,
-                                              const int* err, int bx, int by) {
-    const int i = bx * blockDim.x + threadIdx.x;
-    const int k = by * blockDim.y + threadIdx.y;
-    const int nx = p.nx, nz = p.nz, P = p.P;
-    if (i >= nx || k >= nz || halted(err)) return;
-    const size_t c = MOIST_IDX(k, i);
-    const T rho = a.rho[c];
-    s0[c] = a.q_old[0][c] / rho;
-    s1[c] = a.q_old[1][c] / rho;
-    s2[c] = a.q_old[2][c] / rho;
-    rrho[c] = 1.0 / (double)rho;
-}
-template <class T>
-__global__ void k_stream_prep(DevParams<T> p, TracerArgs<T> a, T* s0, T* s1, T* s2, double* rrho, const int* err) {
-    b_stream_prep(p, a, s0, s1, s2, rrho, err, blockIdx.x, blockIdx.y);
-}
-
-// one tracer t of one domain; blockDim.x = 32 * ceil(nz / 32); ring: [nwarps][2][STREAM_RING]
-template <class T>
-__device__ __forceinline__ void stream_sweep(const DevParams<T>& p, const StreamArgs<T>& a, int t, T* ring) {
-    const int nx = p.nx, nz = p.nz, P = p.P, ke = nz - 1;
-    const int k = threadIdx.x, lane = k & 31, w = k >> 5;
-    const bool row_ok = k < nz;
-    const T* so = a.s_old[t];
-    const T* rho = a.tr.rho;
-    const T* mfx = a.tr.mfx;
-    const T* mfz = a.tr.mfz;
-    const T* q0g = a.tr.q0[t];
-    const T* dphg = a.tr.dphys[t];
-    T* qn = a.tr.q_new[t];
-    const T* qo = a.tr.q_old[t];
-    // stage-start values of row kk at column c (periodic in x), with the padding of the tiled
-    // sweep outside the domain: s = 0, rho = 1, mass fluxes 0
-    auto S = [&](int kk, int c) { return (kk >= 0 && kk < nz) ? so[MOIST_IDX(kk, pmod(c, nx))] : T(0); };
-    auto R = [&](int kk, int c) { return (kk >= 0 && kk < nz) ? rho[MOIST_IDX(kk, pmod(c, nx))] : T(1); };
-    auto MX = [&](int kk, int c) { return (kk >= 0 && kk < nz) ? mfx[MOIST_IDX(kk, pmod(c, nx))] : T(0); };
-    auto MZ = [&](int kk, int c) {
-        return (kk >= 0 && kk < nz && c >= 0 && c < nx) ? mfz[MOIST_IDX(kk, c)] : T(0);
+__device__ __forceinline__ void b_stream_prep(DevParams<T> p, StreamArgs<T> a, const int* err, int bx, int by) {
+    __shared__ T tile[32][34];  // stride 34: a column of an anti-diagonal touches every bank once
+    if (halted(err)) return;  // the same for every thread of the launch
+    const int nx = p.nx, nz = p.nz, P = p.P, np = skew_pitch(nz);
+    const int lane = threadIdx.x & 31, wid = (threadIdx.x + threadIdx.y * blockDim.x) >> 5, nw = (blockDim.x * blockDim.y) >> 5;
+    const int c0 = 32 * bx - 1, k0 = 32 * by;
+    // one field: val(k, i) at the periodic column i of cells (k, c) with c in [c_lo, c_hi]
+    auto field = [&](T* out, int nf, int f, int c_lo, int c_hi, int rows, auto val) {
+        for (int r = wid; r < 32; r += nw) {
+            const int k = k0 + r, c = c0 + lane;
+            tile[r][lane] = (k < rows && c >= c_lo && c <= c_hi) ? val(k, pmod(c, nx)) : T(0);
+        }
+        __syncthreads();
+        for (int d = wid; d < 63; d += nw) {  // anti-diagonal d of the tile: rows r with column d - r
+            const int cc = d - lane, k = k0 + lane, c = c0 + cc;
+            if (cc >= 0 && cc < 32 && k < rows && c >= c_lo && c <= c_hi)
+                out[((size_t)(c + k + 1) * nf + f) * np + k + 1] = tile[lane][cc];
+        }
+        __syncthreads();
     };
+    const T* rho = a.tr.rho;
+    field(a.dom, SK_ND, SK_VX, -1, nx - 1, nz, [&](int k, int i) { return a.tr.mfx[MOIST_IDX(k, i)]; });
+    field(a.dom, SK_ND, SK_VZ, 0, nx - 1, nz - 1, [&](int k, int i) { return a.tr.mfz[MOIST_IDX(k, i)]; });
+    field(a.dom, SK_ND, SK_RX, -1, nx - 1, nz,
+          [&](int k, int i) { return (rho[MOIST_IDX(k, wrapx(i + 1, nx))] + rho[MOIST_IDX(k, i)]) * T(0.5); });
+    field(a.dom, SK_ND, SK_RZ, 0, nx - 1, nz - 1,
+          [&](int k, int i) { return f2h(rho[MOIST_IDX(k + 1, i)], rho[MOIST_IDX(k, i)], p.dz[k + 1], p.dz[k]); });
+    field(a.dom, SK_ND, SK_RHO, 0, nx - 1, nz, [&](int k, int i) { return rho[MOIST_IDX(k, i)]; });
+    field(a.dom, SK_ND, SK_RRHO, 0, nx - 1, nz, [&](int k, int i) { return FastDiv<T>::prep1(rho[MOIST_IDX(k, i)]); });
+    for (int t = 0; t < 3; t++) {
+        field(a.trc[t], SK_NT, SK_S, 0, nx + 1, nz,
+              [&](int k, int i) { return a.tr.q_old[t][MOIST_IDX(k, i)] / rho[MOIST_IDX(k, i)]; });
+        field(a.trc[t], SK_NT, SK_Q0, 0, nx - 1, nz, [&](int k, int i) { return a.tr.q0[t][MOIST_IDX(k, i)]; });
+        field(a.trc[t], SK_NT, SK_DPH, 0, nx - 1, nz, [&](int k, int i) { return a.tr.dphys[t][MOIST_IDX(k, i)]; });
+    }
+}
+template <class T>
+__global__ void __launch_bounds__(256) k_stream_prep(DevParams<T> p, StreamArgs<T> a, const int* err) {
+    b_stream_prep(p, a, err, blockIdx.x, blockIdx.y);
+}
 
-    // row constants (as the tiled sweep forms them)
-    const T dz_k = row_ok ? p.dz[k] : T(1);
-    const T dz_kp1 = (row_ok && k < ke) ? p.dz[k + 1] : T(1);
-    const T dz_km1 = (row_ok && k > 0) ? p.dz[k - 1] : T(1);
-    const T z_k = row_ok ? p.z[k] : T(0);
-    const T z_kp1 = (row_ok && k < ke) ? p.z[k + 1] : T(1);
-    const T z_km1 = (row_ok && k > 0) ? p.z[k - 1] : T(-1);
-    RowRcp<T> rr;
-    rr.dx = T(1) / p.dx;
-    rr.dz_k = T(1) / dz_k;
-    rr.sum_kp = T(1) / (dz_k + dz_kp1);
-    rr.sum_km = T(1) / (dz_km1 + dz_k);
-    rr.zd_kp = T(1) / (z_kp1 - z_k);
-    rr.zd_km = T(1) / (z_k - z_km1);
+__device__ __forceinline__ void cp_async16(void* s, const void* g) {
+    const unsigned sa = (unsigned)__cvta_generic_to_shared(s);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(g) : "memory");
+}
+
+// shared memory of one sweep: the ring of records, then the updated values of the two top rows of
+// every warp ([2][warps][STREAM_RING])
+template <class T>
+__host__ __device__ inline size_t stream_smem_bytes(int nz) {
+    return ((size_t)STREAM_RING * (SK_ND + SK_NT) * skew_pitch(nz) + 2 * ((nz + WROWS - 1) / WROWS) * STREAM_RING) * sizeof(T);
+}
+inline int stream_threads(int nz) { return (nz + WROWS - 1) / WROWS * 32; }
+
+// one tracer t of one domain; blockDim.x = stream_threads(nz) or more. Returns (to every thread)
+// whether the fast division refused an operand or a result is not finite.
+template <class D, class T>
+__device__ __forceinline__ bool stream_sweep(const DevParams<T>& p, const StreamArgs<T>& a, int t, T* smem) {
+    const int nx = p.nx, nz = p.nz, P = p.P, np = skew_pitch(nz);
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nwarp = (nz + WROWS - 1) / WROWS;
+    const int r = lane & (WROWS - 1), k = WROWS * wid + r;
+    const bool zh = lane >= WROWS, row_ok = k < nz;
+    const int recd = SK_ND * np, rect = SK_NT * np, rec = recd + rect;
+    T* top1 = smem + (size_t)STREAM_RING * rec;  // [warp][STREAM_RING]: row 16w+15
+    T* top2 = top1 + nwarp * STREAM_RING;        // row 16w+14
+    const T* gd = a.dom;
+    const T* gt = a.trc[t];
+    constexpr int EPC = 16 / sizeof(T);  // elements per 16-byte copy
+    // record s (>= -1) into its slot of the ring; every thread commits one group per call
+    auto issue = [&](int s) {
+        T* dst = smem + (size_t)((s + 1) & (STREAM_RING - 1)) * rec;
+        const T* sd = gd + (size_t)(s + 1) * recd;
+        const T* st = gt + (size_t)(s + 1) * rect;
+        for (int j = threadIdx.x; j < recd / EPC; j += blockDim.x) cp_async16(dst + j * EPC, sd + j * EPC);
+        for (int j = threadIdx.x; j < rect / EPC; j += blockDim.x) cp_async16(dst + recd + j * EPC, st + j * EPC);
+        cp_async_commit();
+    };
+    const HalfRow<T> w = half_row(p, k, zh, a.tr.dt);
+    const T* qo = a.tr.q_old[t];
     const T lin_km1 = (k - 1 >= 0 && k - 1 < nz) ? qo[MOIST_IDX(k - 1, nx - 2)] : T(0);
     const T lin_k = row_ok ? qo[MOIST_IDX(k, nx - 2)] : T(0);
     const T lin_kp1 = (k + 1 < nz) ? qo[MOIST_IDX(k + 1, nx - 2)] : T(0);
-    FastRow<double> fw{};
-    if constexpr (sizeof(T) == 4) {
-        fw.dx = p.dx;
-        fw.dz_k = dz_k;
-        fw.dz_kp1 = dz_kp1;
-        fw.dz_km1 = dz_km1;
-        fw.sum_kp = dz_k + dz_kp1;
-        fw.sum_km = dz_km1 + dz_k;
-        fw.zd_kp = z_kp1 - z_k;
-        fw.zd_km = z_k - z_km1;
-        fw.rdx = Div64::rcp(fw.dx);
-        fw.rdz_k = Div64::rcp(fw.dz_k);
-        fw.rsum_kp = Div64::rcp(fw.sum_kp);
-        fw.rsum_km = Div64::rcp(fw.sum_km);
-        fw.rzd_kp = Div64::rcp(fw.zd_kp);
-        fw.rzd_km = Div64::rcp(fw.zd_km);
-        fw.kappa = p.kappa;
-        fw.EPS = p.EPS;
-        fw.dt_stage = a.tr.dt;
-        fw.k0 = k == 0;
-        fw.ke = k == ke;
-        fw.kp_at0 = k == 0;
-        fw.kp_atnm2 = k == nz - 2;
-        fw.km_at0 = k - 1 == 0;
-        fw.km_atnm2 = k - 1 == nz - 2;
-    }
-    const bool clamp_kp_row = row_ok && (k == 0 || k == nz - 2) && k < ke;
-    const bool clamp_km_row = row_ok && (k == 1 || k == nz - 1) && k >= 1;
-
-    // the window at the virtual column c = s - k (every thread advances it every step, so that
-    // its neighbours read the right columns before it starts and after it ends). Column indices
-    // of the loads are kept wrapped into [0, nx) incrementally.
-    int c = -k;
-    auto wrap = [&](int x) { return x >= nx ? x - nx : x; };
-    int cw1 = pmod(c + 1, nx), cw2 = pmod(c + 2, nx), cw3 = pmod(c + 3, nx);  // c+1, c+2, c+3 wrapped
-    const bool rin = row_ok, rin_p1 = k + 1 < nz, rin_p2 = k + 2 < nz, rin_m1 = k >= 1 && k - 1 < nz;
-    const T* so_k = so + (size_t)(rin ? k : 0) * P;
-    const T* so_kp1 = so + (size_t)(rin_p1 ? k + 1 : 0) * P;
-    const T* so_kp2 = so + (size_t)(rin_p2 ? k + 2 : 0) * P;
-    const T* rho_k = rho + (size_t)(rin ? k : 0) * P;
-    const T* rho_kp1 = rho + (size_t)(rin_p1 ? k + 1 : 0) * P;
-    const T* rho_km1 = rho + (size_t)(rin_m1 ? k - 1 : 0) * P;
-    const T* mfx_k = mfx + (size_t)(rin ? k : 0) * P;
-    const T* mfz_k = mfz + (size_t)(rin ? k : 0) * P;
-    const T* mfz_km1 = mfz + (size_t)(rin_m1 ? k - 1 : 0) * P;
-    const T* q0_k = q0g + (size_t)(rin ? k : 0) * P;
-    const T* dph_k = dphg + (size_t)(rin ? k : 0) * P;
-    const double* rr_k = a.rrho + (size_t)(rin ? k : 0) * P;
-    const int cw0 = pmod(c, nx), cwm = pmod(c - 1, nx);
-    T s0 = rin ? so_k[cw0] : T(0), s1 = rin ? so_k[cw1] : T(0), s2 = rin ? so_k[cw2] : T(0);
-    T rm = rin ? rho_k[cwm] : T(1), r0 = rin ? rho_k[cw0] : T(1), r1 = rin ? rho_k[cw1] : T(1);
-    T xm = rin ? mfx_k[cwm] : T(0), x0 = rin ? mfx_k[cw0] : T(0);
-    T zp = MZ(k, c - 1), z0 = MZ(k, c);
-    T q0c = rin ? q0_k[cw0] : T(0), dphc = rin ? dph_k[cw0] : T(0);
-    double rrc = rin ? rr_k[cw0] : 1.0;
-    // warp-boundary values of column c: rows k+1, k+2 (top lanes), k-1 (lane 0)
-    T b_s1 = S(k + 1, c), b_s2 = S(k + 2, c), b_r1 = R(k + 1, c), b_rm = R(k - 1, c), b_zm = MZ(k - 1, c);
+    // this half's clamp rows (z half only)
+    const bool clamp_p = zh && row_ok && (k == 0 || k == nz - 2) && k < nz - 1;
+    const bool clamp_m = zh && row_ok && (k == 1 || k == nz - 1) && k >= 1;
     // the updated values of the two columns to the left; the seam reads the stage-start values
-    T prev1 = S(k, nx - 1), prev2 = S(k, nx - 2);
-    T sn_last = T(0), km1_used = T(0);
-    T* top1 = ring;                                    // [w][STREAM_RING]: row 32w+31
-    T* top2 = ring + (blockDim.x >> 5) * STREAM_RING;  // [w][STREAM_RING]: row 32w+30
+    T prev1 = row_ok ? qo[MOIST_IDX(k, nx - 1)] / a.tr.rho[MOIST_IDX(k, nx - 1)] : T(0);
+    T prev2 = row_ok ? qo[MOIST_IDX(k, nx - 2)] / a.tr.rho[MOIST_IDX(k, nx - 2)] : T(0);
+    T sn_last = T(0), m1_used = T(0);
+    T* qn = a.tr.q_new[t] + (size_t)(row_ok ? k : 0) * P;
+    const int z = zh ? 1 : 0, ki = min(k, nz - 1);  // the last warp's rows beyond the domain read row nz-1's inputs
+    const int o_v = (zh ? SK_VZ : SK_VX) * np + ki + 1, o_r = (zh ? SK_RZ : SK_RX) * np + ki + 1;
+    const int o_rho = SK_RHO * np + ki + 1, o_rr = SK_RRHO * np + ki + 1;
+    const int o_s = recd + SK_S * np + ki + 1, o_q = recd + SK_Q0 * np + ki + 1, o_d = recd + SK_DPH * np + ki + 1;
+    const bool in = wid < nwarp;  // warps beyond the rows only copy and meet the barrier
+    bool bad_any = false;
+    struct Ops {
+        T sc, p1, p2, vp, vm, rp, rm, q0, dph, rho, rrho;
+    };
+    auto load = [&](int s) {  // the operands of step s (records s - 1 .. s + 2)
+        auto R = [&](int j) { return smem + (size_t)((j + 1) & (STREAM_RING - 1)) * rec; };
+        const T *R0 = R(s), *Rm = R(s - 1);
+        Ops o;
+        o.sc = R0[o_s];
+        o.p1 = R(s + 1)[o_s + z];
+        o.p2 = R(s + 2)[o_s + 2 * z];
+        o.vp = R0[o_v];
+        o.vm = Rm[o_v - z];
+        o.rp = R0[o_r];
+        o.rm = Rm[o_r - z];
+        o.q0 = R0[o_q];
+        o.dph = R0[o_d];
+        o.rho = R0[o_rho];
+        o.rrho = R0[o_rr];
+        return o;
+    };
 
     const int nsteps = nx + nz - 1;
-    for (int step = 0; step < nsteps; step++, c++) {
-        const bool active = row_ok && c >= 0 && c < nx;
-        // loads for the next column c+1 (one step ahead); mfz only inside the domain
-        const bool zin = c + 1 >= 0 && c + 1 < nx;
-        const T n_s2 = rin ? so_k[cw3] : T(0);
-        const T n_r1 = rin ? rho_k[cw2] : T(1);
-        const T n_x0 = rin ? mfx_k[cw1] : T(0);
-        const T n_z0 = (rin && zin) ? mfz_k[cw1] : T(0);
-        const T n_q0 = rin ? q0_k[cw1] : T(0);
-        const T n_dph = rin ? dph_k[cw1] : T(0);
-        const double n_rr = rin ? rr_k[cw1] : 1.0;
-        T n_bs1 = T(0), n_bs2 = T(0), n_br1 = T(1), n_brm = T(1), n_bzm = T(0);
-        if (lane >= 30) {
-            n_bs1 = rin_p1 ? so_kp1[cw1] : T(0);
-            n_bs2 = rin_p2 ? so_kp2[cw1] : T(0);
-            n_br1 = rin_p1 ? rho_kp1[cw1] : T(1);
-        }
-        if (lane == 0) {
-            n_brm = rin_m1 ? rho_km1[cw1] : T(1);
-            n_bzm = (rin_m1 && zin) ? mfz_km1[cw1] : T(0);
-        }
-        // neighbours: row k-1 stands one column ahead, rows k+1, k+2 one and two behind
-        const T up_sn = __shfl_up_sync(0xffffffffu, sn_last, 1);
-        const T up_km1 = __shfl_up_sync(0xffffffffu, km1_used, 1);
-        const T up_rm = __shfl_up_sync(0xffffffffu, rm, 1);
-        const T up_zp = __shfl_up_sync(0xffffffffu, zp, 1);
-        const T dn_s1 = __shfl_down_sync(0xffffffffu, s1, 1);
-        const T dn_s2 = __shfl_down_sync(0xffffffffu, s2, 2);
-        const T dn_r1 = __shfl_down_sync(0xffffffffu, r1, 1);
-        const int cc = c < 0 ? 0 : (c >= nx ? nx - 1 : c);
-        const T t1 = (w > 0) ? top1[(w - 1) * STREAM_RING + (cc & (STREAM_RING - 1))] : T(0);
-        const T t2 = (w > 0) ? top2[(w - 1) * STREAM_RING + (cc & (STREAM_RING - 1))] : T(0);
-        const T s_km1 = lane == 0 ? t1 : up_sn;
-        const T s_km2 = lane == 0 ? t2 : (lane == 1 ? t1 : up_km1);
-        const T rho_km = lane == 0 ? b_rm : up_rm;
-        const T mfz_km = lane == 0 ? b_zm : up_zp;
-        const T s_kp1 = lane == 31 ? b_s1 : dn_s1;
-        const T s_kp2 = lane >= 30 ? b_s2 : dn_s2;
-        const T rho_kp = lane == 31 ? b_r1 : dn_r1;
-
-        T qn_v = T(0), sn = T(0);
-        if (active) {
-            const size_t cix = MOIST_IDX(k, c);
-            const T q0_c = q0c, dph_c = dphc;
-            // the clamp quotients of limited_flux_z, on the four rows that can use them
-            T cl_kp = T(0), cl_km = T(0);
-            if (clamp_kp_row) cl_kp = z0 > p.EPS ? lin_k / (z0 * p.dt) : lin_kp1 / (-z0 * p.dt);
-            if (clamp_km_row) cl_km = mfz_km > p.EPS ? lin_km1 / (mfz_km * p.dt) : lin_k / (-mfz_km * p.dt);
-#define MOIST_STREAM_IEEE_CELL                                                                            \
-    tracer_cell_t<DivIEEE<T>>(p, k, a.tr.dt, s0, s1, s2, s_kp1, s_kp2, prev1, prev2, s_km1, s_km2, lin_km1,     \
-                              lin_k, lin_kp1, x0, xm, z0, mfz_km, r0, r1, rm, rho_kp, rho_km, dz_k, dz_kp1,       \
-                              dz_km1, z_k, z_kp1, z_km1, q0_c, dph_c, rr, unused)
-            if constexpr (sizeof(T) == 4) {
-                bool bad;
-                unsigned g = ~0u;
-                qn_v = tracer_cell_f<Div64>(fw, s0, s1, s2, s_kp1, s_kp2, prev1, prev2, s_km1, s_km2, cl_kp, cl_km,
-                                            x0, xm, z0, mfz_km, r0, r1, rm, rho_kp, rho_km, q0_c, dph_c, g, bad);
-                sn = Div64::cdiv(qn_v, r0, rrc, g);
-                if (bad || guard_hit(g)) {
-                    unsigned g2 = ~0u;
-                    bool bad2;
-                    qn_v = tracer_cell_f<Div64X>(fw, s0, s1, s2, s_kp1, s_kp2, prev1, prev2, s_km1, s_km2, cl_kp,
-                                                 cl_km, x0, xm, z0, mfz_km, r0, r1, rm, rho_kp, rho_km, q0_c, dph_c,
-                                                 g2, bad2);
-                    sn = Div64X::cdiv(qn_v, r0, rrc, g2);
-                    if (bad2) {
-                        bool unused = false;
-                        qn_v = MOIST_STREAM_IEEE_CELL;
-                        sn = qn_v / r0;
-                    }
-                }
-            } else {
-                bool unused = false;
-                qn_v = MOIST_STREAM_IEEE_CELL;
-                sn = qn_v / r0;
-            }
-#undef MOIST_STREAM_IEEE_CELL
-            qn[cix] = qn_v;
-            if (lane == 31) top1[w * STREAM_RING + (c & (STREAM_RING - 1))] = sn;
-            if (lane == 30) top2[w * STREAM_RING + (c & (STREAM_RING - 1))] = sn;
-            prev2 = prev1;
-            prev1 = sn;
-        }
-        // lane k+1 reads these next step only for the column it shares with this step
-        sn_last = sn;
-        km1_used = s_km1;
-        // advance the window to column c + 1
-        s0 = s1;
-        s1 = s2;
-        s2 = n_s2;
-        rm = r0;
-        r0 = r1;
-        r1 = n_r1;
-        xm = x0;
-        x0 = n_x0;
-        zp = z0;
-        z0 = n_z0;
-        q0c = n_q0;
-        dphc = n_dph;
-        rrc = n_rr;
-        b_s1 = n_bs1;
-        b_s2 = n_bs2;
-        b_r1 = n_br1;
-        b_rm = n_brm;
-        b_zm = n_bzm;
-        cw1 = cw2;
-        cw2 = cw3;
-        cw3 = wrap(cw3 + 1);
+    for (int s = -1; s <= STREAM_RING - 3; s++) issue(s);
+    cp_async_wait<STREAM_RING - 5>();  // records up to 2
+    __syncthreads();
+    Ops nxt = load(0);
+    for (int step = 0; step < nsteps; step++) {
+        // records up to step + 3 have landed (the next step's operands, read one step ahead); the slot of record
+        // step - 2, which nobody reads any more, takes record step + 6 (records beyond the last are allocated)
+        cp_async_wait<STREAM_RING - 6>();
         __syncthreads();
+        issue(step + STREAM_RING - 2);
+        if (!in) continue;
+        const int c = step - k;
+        const bool active = row_ok && c >= 0 && c < nx;
+        const Ops o = nxt;
+        nxt = load(step + 1);
+        // neighbours: row k-1 stands one column ahead
+        const T up_sn = __shfl_up_sync(0xffffffffu, sn_last, 1);
+        const T up_m1 = __shfl_up_sync(0xffffffffu, m1_used, 1);
+        const int slot = c & (STREAM_RING - 1);
+        const T t1 = wid > 0 ? top1[(wid - 1) * STREAM_RING + slot] : T(0);
+        const T t2 = wid > 0 ? top2[(wid - 1) * STREAM_RING + slot] : T(0);
+        const T m1 = zh ? (r == 0 ? t1 : up_sn) : prev1;
+        const T m2 = zh ? (r == 0 ? t2 : (r == 1 ? t1 : up_m1)) : prev2;
+        T q, sn;
+        bool bad = false;
+        if (__any_sync(0xffffffffu, active && (clamp_p || clamp_m || !(fabs(o.vp) > w.EPS) || !(fabs(o.vm) > w.EPS)))) {
+            // the clamp quotients of limited_flux_z, on the four rows that can use them
+            T cl_p = T(0), cl_m = T(0);
+            if (clamp_p) cl_p = o.vp > w.EPS ? lin_k / (o.vp * p.dt) : lin_kp1 / (-o.vp * p.dt);
+            if (clamp_m) cl_m = o.vm > w.EPS ? lin_km1 / (o.vm * p.dt) : lin_k / (-o.vm * p.dt);
+            two_lane_cell<D, true>(w, m2, m1, o.sc, o.p1, o.p2, o.vp, o.vm, o.rp, o.rm, cl_p, cl_m, o.q0, o.dph, o.rho,
+                                   o.rrho, q, sn, bad);
+        } else {
+            two_lane_cell<D, false>(w, m2, m1, o.sc, o.p1, o.p2, o.vp, o.vm, o.rp, o.rm, T(0), T(0), o.q0, o.dph, o.rho,
+                                    o.rrho, q, sn, bad);
+        }
+        bad_any |= bad && active;
+        if (active && !zh) {
+            qn[c] = q;
+            if (r == WROWS - 1) top1[wid * STREAM_RING + slot] = sn;
+            if (r == WROWS - 2) top2[wid * STREAM_RING + slot] = sn;
+        }
+        prev2 = active ? prev1 : prev2;
+        prev1 = active ? sn : prev1;
+        // lane r+1 reads these next step only for the column it shares with this step
+        sn_last = sn;
+        m1_used = m1;
     }
+    cp_async_wait<0>();
+    return __syncthreads_or(bad_any) != 0;
 }
 
-// tracer t of one domain (the block's threads: 32 * ceil(nz / 32) or more)
+// tracer t of one domain
 template <class T>
 __device__ __forceinline__ void b_tracer_stream(const DevParams<T>& p, const StreamArgs<T>& a, const int* err, int t) {
-    __shared__ T ring[2 * (STREAM_MAX_ROWS / 32) * STREAM_RING];
+    extern __shared__ __align__(16) unsigned char smem_raw[];
     if (halted(err)) return;
-    stream_sweep(p, a, t, ring);
+    T* sm = reinterpret_cast<T*>(smem_raw);
+    if (stream_sweep<FastDiv<T>>(p, a, t, sm)) stream_sweep<IeeeDiv<T>>(p, a, t, sm);
 }
 
 // single domain: block t sweeps tracer t
 template <class T>
-__global__ void __launch_bounds__(STREAM_MAX_ROWS) k_tracer_stream(DevParams<T> p, StreamArgs<T> a, const int* err) {
+__global__ void __launch_bounds__(2 * STREAM_MAX_ROWS) k_tracer_stream(DevParams<T> p, StreamArgs<T> a, const int* err) {
     b_tracer_stream(p, a, err, blockIdx.x);
 }
 
