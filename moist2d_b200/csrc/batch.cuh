@@ -54,7 +54,8 @@ struct BRd {
     DevParams<T> p;
     StateP<T> s;
     const T* theta_ref;
-    T *lw_up, *lw_dn, *d_th_rd;
+    T* d_th_rd;
+    int wc;
     const int* err;
 };
 template <class T>
@@ -144,7 +145,7 @@ struct FSf {
 template <class T>
 struct FRd {
     __device__ void operator()(const BRd<T>& a, int bx, int by) const {
-        b_gray_radiation(a.p, a.s, a.theta_ref, a.lw_up, a.lw_dn, a.d_th_rd, a.err, bx, by);
+        b_gray_radiation(a.p, a.s, a.theta_ref, a.d_th_rd, a.wc, a.err, bx, by);
     }
 };
 template <class T>

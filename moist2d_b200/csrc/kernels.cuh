@@ -87,60 +87,105 @@ __device__ __forceinline__ T tanh_m(T x) {  // tanh from the shared exp
     return (e - T(1)) / (e + T(1));
 }
 
-// gray_radiation! (moist.jl:776-840), one thread per column; LW_up / LW_dn scratch [nz+1][P]
+// gray_radiation! (moist.jl:776-840) over a strip of wc adjacent columns per block of RD_THREADS
+// threads. The cell quantities (a power and an exponential in double precision each) are formed
+// once for all cells in parallel, the two flux recurrences (up on one thread per column, down on
+// another) run out of shared memory, the heating rates over all cells again. One thread per column
+// formed every cell's powers three times in the order of the recurrences: 1.38 ms for 640 x 250
+// (Float32; 20 warps on the GPU), 0.04 ms this way. wc: 8, or fewer where 148 blocks or the shared
+// memory of two blocks per SM ask for it (rd_strip).
+constexpr int RD_THREADS = 256;
 template <class T>
-__device__ __forceinline__ void b_gray_radiation(DevParams<T> p, StateP<T> s, const T* theta_ref, T* lw_up, T* lw_dn,
-                                                 T* d_th_rd, const int* err, int bx, int by) {
-    const int i = bx * blockDim.x + threadIdx.x;
+__host__ __device__ inline size_t rd_smem_bytes(int nz, int wc) {
+    return ((size_t)3 * nz + 2 * (size_t)(nz + 1)) * wc * sizeof(T);
+}
+template <class T>
+inline int rd_strip(int nx, int nz, int nsm) {
+    for (int w : {8, 4, 2})
+        if ((nx + w - 1) / w >= nsm && rd_smem_bytes<T>(nz, w) <= 96 * 1024) return w;
+    return 1;
+}
+template <class T>
+__device__ __forceinline__ void b_gray_radiation(DevParams<T> p, StateP<T> s, const T* theta_ref, T* d_th_rd, int wc,
+                                                 const int* err, int bx, int by) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    if (halted(err)) return;  // the same for every thread of the launch
     const int nx = p.nx, nz = p.nz, P = p.P;
-    if (i >= nx || halted(err)) return;
-    auto col = [&](int k, T& cpk, T& pik, T& tempk, T& epsk, T& tauk) {
-        const size_t c = MOIST_IDX(k, i);
+    const int i0 = bx * wc, ncol = min(wc, nx - i0);
+    const size_t n = (size_t)nz * wc;
+    T* tau = reinterpret_cast<T*>(smem_raw);  // [nz][wc] transmissivity
+    T* em = tau + n;                          // emission eps sigma T^4
+    T* cpi = em + n;                          // cp Pi
+    T* up = cpi + n;                          // [nz+1][wc] upward flux at the faces
+    T* dn = up + n + wc;                      // downward flux
+    for (int e = threadIdx.x; e < nz * wc; e += blockDim.x) {
+        const int k = e / wc, col = e - k * wc;
+        if (col >= ncol) continue;
+        const size_t c = MOIST_IDX(k, i0 + col);
         const T rho = s.rho[c];
         const T qv = s.qv[c] / rho, qc = s.qc[c] / rho, qr = s.qr[c] / rho;
         const T qd = T(1.0) - qv - qc - qr;
         const T r = p.Rd * qd + p.Rv * qv;
-        cpk = p.Cpd * qd + p.Cpv * qv + p.Cpl * (qc + qr);
+        const T cpk = p.Cpd * qd + p.Cpv * qv + p.Cpl * (qc + qr);
         const T cv = cpk - r;
-        pik = mm::mpow(r * s.rt[c] / p.P0, r / cv);
-        tempk = s.rt[c] / rho * pik;
+        const T pik = mm::mpow(r * s.rt[c] / p.P0, r / cv);
+        const T tempk = s.rt[c] / rho * pik;
         const T dq = p.k_abs_qv * s.qv[c] * p.dz[k];
         const T dc = p.k_abs_qc * s.qc[c] * p.dz[k];
         const T dr = p.k_abs_qr * s.qr[c] * p.dz[k];
-        epsk = T(1.0) - mm::mexp(-(dq + dc + dr));
-        tauk = T(1.0) - epsk;
-    };
-    T cpk, pik, tempk, epsk, tauk;
-    T up = p.surf_emissivity * p.SIGMA * mm::mpow4(p.temp_surf);
-    lw_up[MOIST_IDX(0, i)] = up;
-    for (int k = 0; k < nz; k++) {
-        col(k, cpk, pik, tempk, epsk, tauk);
-        up = up * tauk + epsk * p.SIGMA * mm::mpow4(tempk);
-        lw_up[MOIST_IDX(k + 1, i)] = up;
+        const T epsk = T(1.0) - mm::mexp(-(dq + dc + dr));
+        tau[e] = T(1.0) - epsk;
+        em[e] = epsk * p.SIGMA * mm::mpow4(tempk);
+        cpi[e] = cpk * pik;
     }
-    T dn = T(0.0);
-    lw_dn[MOIST_IDX(nz, i)] = dn;
-    for (int k = nz - 1; k >= 0; k--) {
-        col(k, cpk, pik, tempk, epsk, tauk);
-        dn = dn * tauk + epsk * p.SIGMA * mm::mpow4(tempk);
-        lw_dn[MOIST_IDX(k, i)] = dn;
+    __syncthreads();
+    if (threadIdx.x < ncol) {
+        const int c = threadIdx.x;
+        T f = p.surf_emissivity * p.SIGMA * mm::mpow4(p.temp_surf);
+        up[c] = f;
+        T t = tau[c], m = em[c];
+#pragma unroll 4
+        for (int k = 0; k < nz; k++) {  // the next level's operands are read one level ahead
+            const int kn = min(k + 1, nz - 1);
+            const T tn = tau[kn * wc + c], mn = em[kn * wc + c];
+            f = f * t + m;
+            up[(k + 1) * wc + c] = f;
+            t = tn;
+            m = mn;
+        }
+    } else if (threadIdx.x >= 32 && threadIdx.x < 32 + ncol) {
+        const int c = threadIdx.x - 32;
+        T f = T(0.0);
+        dn[nz * wc + c] = f;
+        T t = tau[(nz - 1) * wc + c], m = em[(nz - 1) * wc + c];
+#pragma unroll 4
+        for (int k = nz - 1; k >= 0; k--) {
+            const int kn = max(k - 1, 0);
+            const T tn = tau[kn * wc + c], mn = em[kn * wc + c];
+            f = f * t + m;
+            dn[k * wc + c] = f;
+            t = tn;
+            m = mn;
+        }
     }
+    __syncthreads();
     const T dz_trans = T(2.0e3);
-    for (int k = 0; k < nz; k++) {
-        col(k, cpk, pik, tempk, epsk, tauk);
-        const T divF = ((lw_up[MOIST_IDX(k + 1, i)] - lw_dn[MOIST_IDX(k + 1, i)]) -
-                        (lw_up[MOIST_IDX(k, i)] - lw_dn[MOIST_IDX(k, i)])) / p.dz[k];
-        const T hr = -divF / (cpk * pik);
+    for (int e = threadIdx.x; e < nz * wc; e += blockDim.x) {
+        const int k = e / wc, col = e - k * wc;
+        if (col >= ncol) continue;
+        const T divF = ((up[e + wc] - dn[e + wc]) - (up[e] - dn[e])) / p.dz[k];
+        const T hr = -divF / cpi[e];
         const T alpha = T(0.5) * (T(1.0) + tanh_m((p.z[k] - (p.z_trop + dz_trans * T(0.5))) / dz_trans)) /
                         p.tau_cooling;
-        const size_t c = MOIST_IDX(k, i);
+        const size_t c = MOIST_IDX(k, i0 + col);
         const T cr = -(s.rt[c] - s.rho[c] * theta_ref[k]) * alpha;
         d_th_rd[c] = hr + cr;
     }
 }
 template <class T>
-__global__ void k_gray_radiation(DevParams<T> p, StateP<T> s, const T* theta_ref, T* lw_up,                                  T* lw_dn, T* d_th_rd, const int* err) {
-    b_gray_radiation(p, s, theta_ref, lw_up, lw_dn, d_th_rd, err, blockIdx.x, blockIdx.y);
+__global__ void __launch_bounds__(RD_THREADS) k_gray_radiation(DevParams<T> p, StateP<T> s, const T* theta_ref,
+                                                               T* d_th_rd, int wc, const int* err) {
+    b_gray_radiation(p, s, theta_ref, d_th_rd, wc, err, blockIdx.x, blockIdx.y);
 }
 
 // Kessler microphysics + rain sedimentation + assembly of the six phys tendencies

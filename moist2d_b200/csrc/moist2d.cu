@@ -217,7 +217,7 @@ struct Ctx : CtxBase {
     StateP<T> cur, nxt, s0b;
     T* tmpq[3];
     PhysP<T> ph;
-    T *d_th_mp, *d_qv_mp, *d_qc_mp, *d_qr_mp, *d_qr_sed, *d_th_rd, *lw_up, *lw_dn;
+    T *d_th_mp, *d_qv_mp, *d_qc_mp, *d_qr_mp, *d_qr_sed, *d_th_rd;
     T *pres, *theta, *rt2p, *uface, *wface, *R_rho, *R_ru, *R_rw, *R_rt;
     T *rho_p, *ru_p[2], *rw_p, *rt_p[3], *mfx, *mfz, *ta, *tb, *tc;
     TT *tcp, *tpiv, *dprime;
@@ -230,6 +230,7 @@ struct Ctx : CtxBase {
     CSum* bud_part;   // [BUDGET_BLOCKS][4] block sums of the budgets
     double* bud_res;  // [4]
     bool rd_dirty = true;
+    bool sf_dirty = true;  // the surface fluxes and tendencies may hold something else than zero
     // tiled tracer sweep (tracer_tiles.cuh)
     bool use_tiles = false;
     bool tiles_df = false;  // the tiled sweep without grid barriers (per-tile versions)
@@ -246,6 +247,7 @@ struct Ctx : CtxBase {
     // column strips of the factorisation and the acoustic substeps
     int strip_wc = 1;
     size_t strip_smem = 0;
+    int rd_wc = 1;  // columns per block of the radiation
     // adjoint tape: when set, run_stage copies the stage internals the reverse sweep needs
     struct Tape {
         T* in[3][7];                           // stage inputs
@@ -365,8 +367,6 @@ struct Ctx : CtxBase {
                       &ru_p[0], &ru_p[1], &rw_p, &rt_p[0], &rt_p[1], &rt_p[2], &mfx, &mfz, &ta, &tb, &tc})
             AL(*f, fsz);
         s0b = StateP<T>{nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
-        AL(lw_up, (size_t)(nz + 1) * P);
-        AL(lw_dn, (size_t)(nz + 1) * P);
         AL(tcp, fsz);
         AL(tpiv, fsz);
         AL(dprime, fsz);
@@ -465,6 +465,8 @@ struct Ctx : CtxBase {
         CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
         CK(cudaFuncSetAttribute(k_thomas_strip<T, TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
         CK(cudaFuncSetAttribute(k_substep_strip<T, TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
+        rd_wc = rd_strip<T>(nx, nz, nsm);
+        CK(cudaFuncSetAttribute(k_gray_radiation<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
         return MOIST_OK;
     }
 
@@ -665,6 +667,7 @@ struct Ctx : CtxBase {
         for (int j = 0; j < 6; j++)
             if ((r = put2d(g2[j], gv[j])) != MOIST_OK) return r;
         if (s->d_rho_theta_rd) rd_dirty = true;
+        sf_dirty = true;
         const void* f1[8] = {s->prec, s->mflux, s->shflux, s->lhflux, s->d_rho_u_sf, s->d_rho_theta_sf,
                              s->d_rho_qv_sf, nullptr};
         T* d1[8] = {prec, mflux, shflux, lhflux, d_u_sf, d_th_sf, d_qv_sf, nullptr};
@@ -724,19 +727,19 @@ struct Ctx : CtxBase {
                                                                       d_th_sf, d_qv_sf, mflux, shflux, lhflux, err);
                     CKL();
                 }
-            } else {
-                for (T* f : {d_u_sf, d_th_sf, d_qv_sf, mflux, shflux, lhflux}) {
-                    if (rec)
-                        rec->put(BK_MEMSET, BMemset{f, P * sizeof(T)});
-                    else
-                        CK(cudaMemsetAsync(f, 0, P * sizeof(T), st));
-                }
+            } else if (rec) {  // a recorded step clears every time: uploads may come between steps
+                for (T* f : {d_u_sf, d_th_sf, d_qv_sf, mflux, shflux, lhflux})
+                    rec->put(BK_MEMSET, BMemset{f, P * sizeof(T)});
+            } else if (sf_dirty) {
+                for (T* f : {d_u_sf, d_th_sf, d_qv_sf, mflux, shflux, lhflux}) CK(cudaMemsetAsync(f, 0, P * sizeof(T), st));
+                sf_dirty = false;
             }
             if (dp.do_rd) {
                 if (rec) {
-                    rec->put(BK_RD, BRd<T>{dp, cur, theta_ref, lw_up, lw_dn, d_th_rd, err});
+                    rec->put(BK_RD, BRd<T>{dp, cur, theta_ref, d_th_rd, rd_wc, err});
                 } else {
-                    k_gray_radiation<T><<<cdiv(nx, 128), 128, 0, st>>>(dp, cur, theta_ref, lw_up, lw_dn, d_th_rd, err);
+                    k_gray_radiation<T><<<cdiv(nx, rd_wc), RD_THREADS, rd_smem_bytes<T>(nz, rd_wc), st>>>(dp, cur, theta_ref,
+                                                                                                    d_th_rd, rd_wc, err);
                     CKL();
                 }
                 rd_dirty = true;
@@ -1148,6 +1151,7 @@ struct Ctx : CtxBase {
     int surface_fluxes() override {
         if (halo < 1) return set_err(owner, MOIST_ERR_ARG, "surface_fluxes! reads one halo column: halo >= 1");
         CK(reset_err());
+        sf_dirty = true;
         k_surface_fluxes<T><<<cdiv(nx, 128), 128, 0, st>>>(dp, cur, halo_vals, halo_vals + 1, d_u_sf, d_th_sf,
                                                           d_qv_sf, mflux, shflux, lhflux, err);
         CKL();
@@ -1157,7 +1161,8 @@ struct Ctx : CtxBase {
     // gray_radiation! (moist.jl:776-840) on the current state alone, with the uploaded theta_ref
     int gray_radiation() override {
         CK(reset_err());
-        k_gray_radiation<T><<<cdiv(nx, 128), 128, 0, st>>>(dp, cur, theta_ref, lw_up, lw_dn, d_th_rd, err);
+        k_gray_radiation<T><<<cdiv(nx, rd_wc), RD_THREADS, rd_smem_bytes<T>(nz, rd_wc), st>>>(dp, cur, theta_ref,
+                                                                                                    d_th_rd, rd_wc, err);
         CKL();
         rd_dirty = true;
         return finish();
@@ -2021,8 +2026,15 @@ struct BatchImpl : BatchBase {
                 for (int i = 0; i < n; i++)
                     if (in_group(i)) it.push_back({i, 0, 0});
                 break;
-            case BK_SF:
             case BK_RD:
+                block = dim3(RD_THREADS);
+                for (int i = 0; i < n; i++)
+                    if (in_group(i)) {
+                        smem = std::max(smem, rd_smem_bytes<T>(m[i]->nz, m[i]->rd_wc));
+                        for (unsigned bx = 0; bx < cdiv(m[i]->nx, m[i]->rd_wc); bx++) it.push_back({i, (int)bx, 0});
+                    }
+                break;
+            case BK_SF:
             case BK_PREC:
                 block = dim3(128);
                 for (int i = 0; i < n; i++)
@@ -2554,6 +2566,7 @@ struct BatchImpl : BatchBase {
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
             BCK(cudaFuncSetAttribute(k_batched<SINGLE_ARG(BSub<T, TT>), SINGLE_ARG(FSubAsync<T, TT, 3>), 2>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
+            BCK(cudaFuncSetAttribute(k_batched<BRd<T>, FRd<T>, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
             BCK(cudaFuncSetAttribute(k_batched_b<BStream<T>, FStream<T>, 2 * STREAM_MAX_ROWS, 1>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
             BCK(cudaFuncSetAttribute(k_batched_b<BStream<T>, FStream<T>, 256, 2>,
