@@ -8,35 +8,27 @@
 // keeps other streams busy cannot afford cudaFree, which waits for the whole device.
 // moist_implicit_correction allocates its column buffers on every call; this variant
 // allocates nothing. The grid vectors travel in the kernel's parameter block (so the call
-// issues no host-to-device copy either), and the scratch of the elimination (the modified
-// super-diagonal and right-hand side of every column) lives in one file-scope __device__ array
-// of fixed size that every GPU loading the library holds until the process exits.
+// issues no host-to-device copy either), and the elimination works in shared memory.
 #include <cuda_runtime.h>
 
 #include <cstdio>
 #include <cstring>
-#include <mutex>
 
 #include "../../include/moist2d.h"
+#include "fastdiv.cuh"
 #include "model.cuh"
 
 namespace {
 
-constexpr size_t kScratchDoubles = MOIST_NOALLOC_SCRATCH_BYTES / sizeof(double);
-static __device__ __align__(256) double g_noalloc_scratch[kScratchDoubles];
-
 // the grid vectors dz and z, passed by value in the kernel's parameter block (at most
-// MOIST_NOALLOC_MAX_NZ levels: 16 KiB in Float64, within the 32 KiB parameter limit)
-template <class T>
+// MOIST_NOALLOC_MAX_NZ levels: 16 KiB in Float64, within the 32 KiB parameter limit). The smaller of two
+// capacities that holds nz travels: 16 KiB of parameters a launch cost the host and the GPU's front
+// end more than the solve of a small call.
+template <class T, int CAP>
 struct ColumnGrid {
-    T dz[MOIST_NOALLOC_MAX_NZ];
-    T z[MOIST_NOALLOC_MAX_NZ];
+    T dz[CAP];
+    T z[CAP];
 };
-
-// device address of g_noalloc_scratch, looked up once per device with that device current
-constexpr int kMaxDevices = 64;
-void* g_scratch_addr[kMaxDevices] = {nullptr};
-std::mutex g_scratch_mutex;
 
 void put_msg(char* err, size_t errlen, const char* msg) {
     if (err && errlen) {
@@ -45,69 +37,151 @@ void put_msg(char* err, size_t errlen, const char* msg) {
     }
 }
 
-// one thread per column; column j of each (nz, ncols) array starts at j * nz (z fastest, the
-// reference layout). Same arithmetic as implicit_correction! (moist.jl:974-1030) and
-// solve_tridiagonal! (moist.jl:952-971), with the elimination in TT.
+// shared memory of one level of one column: a, b + 1, c, d (T), c', d' (TT)
 template <class T, class TT>
-__global__ void k_implicit_columns_noalloc(int nz, int ncols, T grav, T beta, T* rho_w, const T* drho_w,
-                                          const T* theta, const T* rt2pres, T dt,
-                                          const __grid_constant__ ColumnGrid<T> grid, TT* work) {
-    const int j = blockIdx.x * blockDim.x + threadIdx.x;
-    if (j >= ncols) return;
-    const T* dz = grid.dz;  // every thread reads the same level at the same time: broadcast
-    const T* z = grid.z;
-    const int n = nz - 1, ke = nz - 1;
-    T* w = rho_w + (size_t)j * nz;
-    const T* dw = drho_w + (size_t)j * nz;
-    const T* th = theta + (size_t)j * nz;
-    const T* r2 = rt2pres + (size_t)j * nz;
-    TT* cps = work + (size_t)j * 2 * n;
-    TT* dps = cps + n;
+constexpr size_t level_bytes() {
+    return 4 * sizeof(T) + 2 * sizeof(TT);
+}
+// elements from one column to the next: odd, so that the columns' threads read different banks
+__host__ __device__ inline int column_stride(int nz, int wc) { return wc == 1 ? nz : (nz | 1); }
+constexpr int kThreads = 128;
+
+// wc adjacent columns per block, column j of each (nz, ncols) array starting at j * nz (z fastest, the
+// reference layout): a block's columns are one contiguous piece of every array. All threads form the
+// coefficients and right-hand sides of the piece's levels (whole-line loads, divisions in
+// parallel), one thread per column eliminates and substitutes in shared memory, all threads write the
+// piece back. What bounds it is the elimination's chain: two multiply-subtracts and the
+// quotients c' and d' per level, both from one reciprocal of the pivot (rcp_rn and two remainder
+// corrections, fastdiv.cuh; a column with a refused or non-finite quotient is eliminated again with
+// IEEE division). Same arithmetic as implicit_correction! (moist.jl:974-1030) and solve_tridiagonal!
+// (moist.jl:952-971), with the elimination in TT. One thread per column out of global memory, every
+// load a line of its own: 204 us for 2048 columns of 128 levels (Float32, FP64 elimination).
+template <class T, class TT, int CAP>
+__global__ void __launch_bounds__(kThreads) k_implicit_columns_noalloc(int nz, int ncols, int wc, T grav, T beta, T* rho_w,
+                                                                       const T* drho_w, const T* theta,
+                                                                       const T* rt2pres, T dt,
+                                                                       const __grid_constant__ ColumnGrid<T, CAP> grid) {
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    using F = moist::FastDiv<TT>;
+    const int n = nz - 1, ke = nz - 1, ld = column_stride(nz, wc);
+    const int j0 = blockIdx.x * wc, nc = min(wc, ncols - j0);
+    TT* cps = reinterpret_cast<TT*>(smem_raw);  // [wc][ld]
+    TT* dps = cps + (size_t)wc * ld;
+    T* sa = reinterpret_cast<T*>(dps + (size_t)wc * ld);
+    T* sb = sa + (size_t)wc * ld;
+    T* sc = sb + (size_t)wc * ld;
+    T* sd = sc + (size_t)wc * ld;
     const T fact_tp = T(0.5) * (T(1.0) + beta);
     const T fact_tm = T(0.5) * (T(1.0) - beta);
     const T dt_tp2 = (dt * fact_tp) * (dt * fact_tp);
     const T fact = fact_tm / fact_tp;
-    TT cp_prev = TT(0), d_prev = TT(0);
-    for (int k = 0; k < n; k++) {
-        const T th_cur = moist::f2h(th[k], th[k + 1], dz[k], dz[k + 1]);
-        const T th_prev = k > 0 ? moist::f2h(th[k - 1], th[k], dz[k - 1], dz[k]) : T(0);
-        const T th_next = (k + 1 <= ke - 1) ? moist::f2h(th[k + 1], th[k + 2], dz[k + 1], dz[k + 2]) : T(0);
-        const T b = dt_tp2 * (r2[k] / dz[k] + r2[k + 1] / dz[k + 1]) * th_cur / (z[k + 1] - z[k]);
-        const T a = (k > 0) ? -dt_tp2 * (r2[k] * th_prev / ((z[k + 1] - z[k]) * dz[k]) - grav / (dz[k] + dz[k + 1])) : T(0);
-        const T c = (k < ke - 1) ? -dt_tp2 * (r2[k + 1] * th_next / ((z[k + 1] - z[k]) * dz[k + 1]) + grav / (dz[k] + dz[k + 1])) : T(0);
-        T d = w[k] + dw[k];
-        if (k > 0) d -= a * fact * w[k];
-        d -= b * fact * w[k];
-        const T bb = b + T(1.0);
-        if (k < ke - 1) d -= c * fact * w[k + 1];
-        TT piv, cpk, dpk;
-        if (k == 0) {
-            piv = (TT)bb;
-            cpk = (TT)c / piv;
-            dpk = (TT)d / piv;
-        } else {
-            piv = (TT)bb - (TT)a * cp_prev;
-            cpk = (TT)c / piv;
-            dpk = ((TT)d - (TT)a * d_prev) / piv;
+    const size_t base = (size_t)j0 * nz;
+    for (int e = threadIdx.x; e < nc * nz; e += kThreads) {
+        const int col = e / nz, k = e - col * nz;
+        if (k >= n) continue;
+        const int o = col * ld + k;
+        const T* th = theta + base + e;    // this level of this column
+        const T* r2 = rt2pres + base + e;
+        const T* w = rho_w + base + e;
+        const T dz_k = grid.dz[k], dz_kp = grid.dz[k + 1], zd = grid.z[k + 1] - grid.z[k];
+        const T th_cur = moist::f2h(th[0], th[1], dz_k, dz_kp);
+        const T th_prev = k > 0 ? moist::f2h(th[-1], th[0], grid.dz[k - 1], dz_k) : T(0);
+        const T th_next = (k + 1 <= ke - 1) ? moist::f2h(th[1], th[2], dz_kp, grid.dz[k + 2]) : T(0);
+        const T b = dt_tp2 * (r2[0] / dz_k + r2[1] / dz_kp) * th_cur / zd;
+        const T a = (k > 0) ? -dt_tp2 * (r2[0] * th_prev / (zd * dz_k) - grav / (dz_k + dz_kp)) : T(0);
+        const T c = (k < ke - 1) ? -dt_tp2 * (r2[1] * th_next / (zd * dz_kp) + grav / (dz_k + dz_kp)) : T(0);
+        T d = w[0] + drho_w[base + e];
+        if (k > 0) d -= a * fact * w[0];
+        d -= b * fact * w[0];
+        if (k < ke - 1) d -= c * fact * w[1];
+        sa[o] = a;
+        sb[o] = b + T(1.0);
+        sc[o] = c;
+        sd[o] = d;
+    }
+    __syncthreads();
+    if (threadIdx.x < nc) {
+        const size_t o = (size_t)threadIdx.x * ld;
+        const T* __restrict__ pa = sa + o;
+        const T* __restrict__ pb = sb + o;
+        const T* __restrict__ pc = sc + o;
+        T* __restrict__ pd = sd + o;
+        TT* __restrict__ cp = cps + o;
+        TT* __restrict__ dp = dps + o;
+        auto eliminate = [&](auto quotients) {
+            TT c_prev = TT(0), d_prev = TT(0);
+            T an = pa[0], bn = pb[0], cn = pc[0], dn = pd[0];
+#pragma unroll 2
+            for (int k = 0; k < n; k++) {  // the next level's operands are read one level ahead
+                const TT a = (TT)an, b = (TT)bn, c = (TT)cn, d = (TT)dn;
+                const int kn = k + 1 < n ? k + 1 : n - 1;
+                an = pa[kn];
+                bn = pb[kn];
+                cn = pc[kn];
+                dn = pd[kn];
+                const TT piv = k == 0 ? b : b - a * c_prev, num = k == 0 ? d : d - a * d_prev;
+                quotients(c, num, piv, c_prev, d_prev);
+                cp[k] = c_prev;
+                dp[k] = d_prev;
+            }
+        };
+        bool bad = false;
+        eliminate([&](TT c, TT num, TT piv, TT& q_c, TT& q_d) {
+            bad |= !(piv >= F::LO && piv <= F::HI);
+            const TT y = moist::rcp_rn(piv, bad);
+            q_c = F::twice(c, piv, y, piv * F::TIE, bad);
+            q_d = F::twice(num, piv, y, piv * F::TIE, bad);
+            bad |= !(fabs(q_c) <= F::MAX) || !(fabs(q_d) <= F::MAX);
+        });
+        if (bad)
+            eliminate([&](TT c, TT num, TT piv, TT& q_c, TT& q_d) {
+                q_c = c / piv;
+                q_d = num / piv;
+            });
+        TT x = dp[n - 1];
+        pd[n - 1] = (T)x;
+        const int k1 = n >= 2 ? n - 2 : 0;
+        TT dn = dp[k1], cn = cp[k1];
+#pragma unroll 4
+        for (int k = n - 2; k >= 0; k--) {
+            const TT dk = dn, ck = cn;
+            const int kn = k >= 1 ? k - 1 : 0;
+            dn = dp[kn];
+            cn = cp[kn];
+            x = dk - ck * x;
+            pd[k] = (T)x;
         }
-        cps[k] = cpk;
-        dps[k] = dpk;
-        cp_prev = cpk;
-        d_prev = dpk;
     }
-    TT x = dps[n - 1];
-    w[n - 1] = (T)x;
-    for (int k = n - 2; k >= 0; k--) {
-        x = dps[k] - cps[k] * x;
-        w[k] = (T)x;
+    __syncthreads();
+    for (int e = threadIdx.x; e < nc * nz; e += kThreads) {
+        const int col = e / nz, k = e - col * nz;
+        if (k < n) rho_w[base + e] = sd[col * ld + k];  // the lid face is never solved
     }
+}
+
+template <class T, class TT, int CAP>
+cudaError_t launch_noalloc(const moist_params* p, int ncols, void* rho_w, const void* drho_w, const void* theta,
+                           const void* rt2pres, double dt, cudaStream_t st) {
+    const int nz = p->nz;
+    ColumnGrid<T, CAP> grid;  // levels from nz on are never read
+    std::memcpy(grid.dz, p->dz, nz * sizeof(T));
+    std::memcpy(grid.z, p->z, nz * sizeof(T));
+    // columns per block: 8, fewer where the default 48 KiB of shared memory ask for it (one column of 1024
+    // levels takes 48 KiB in Float64) or while the blocks are fewer than the SMs, whose chains run side by side
+    auto bytes = [&](int w) { return level_bytes<T, TT>() * column_stride(nz, w) * w; };
+    int wc = 8;
+    while (wc > 1 && (bytes(wc) > 48 * 1024 || (ncols + wc - 1) / wc < 148)) wc /= 2;
+    k_implicit_columns_noalloc<T, TT, CAP><<<(ncols + wc - 1) / wc, kThreads, bytes(wc), st>>>(
+        nz, ncols, wc, (T)p->grav, (T)p->beta_offcenter, (T*)rho_w, (const T*)drho_w, (const T*)theta,
+        (const T*)rt2pres, (T)dt, grid);
+    return cudaGetLastError();
 }
 
 template <class T, class TT>
 int run_noalloc(const moist_params* p, int ncols, void* rho_w, const void* drho_w, const void* theta,
-                const void* rt2pres, double dt, cudaStream_t st, double* base, char* err, size_t errlen) {
+                const void* rt2pres, double dt, cudaStream_t st, char* err, size_t errlen) {
     const int nz = p->nz;
-    // scratch: the elimination work (TT, 2 (nz-1) per column)
+    // the call's documented limit: the elimination's values (TT, 2 (nz-1) per column)
     const size_t work_bytes = 2 * (size_t)(nz - 1) * ncols * sizeof(TT);
     if (work_bytes > MOIST_NOALLOC_SCRATCH_BYTES) {
         char msg[256];
@@ -118,16 +192,8 @@ int run_noalloc(const moist_params* p, int ncols, void* rho_w, const void* drho_
         put_msg(err, errlen, msg);
         return MOIST_ERR_ARG;
     }
-    ColumnGrid<T> grid;
-    std::memset(&grid, 0, sizeof grid);
-    std::memcpy(grid.dz, p->dz, nz * sizeof(T));
-    std::memcpy(grid.z, p->z, nz * sizeof(T));
-    TT* work = reinterpret_cast<TT*>(base);
-    const int threads = 128;
-    k_implicit_columns_noalloc<T, TT><<<(ncols + threads - 1) / threads, threads, 0, st>>>(
-        nz, ncols, (T)p->grav, (T)p->beta_offcenter, (T*)rho_w, (const T*)drho_w, (const T*)theta,
-        (const T*)rt2pres, (T)dt, grid, work);
-    cudaError_t e = cudaGetLastError();
+    const cudaError_t e = nz <= 256 ? launch_noalloc<T, TT, 256>(p, ncols, rho_w, drho_w, theta, rt2pres, dt, st)
+                                    : launch_noalloc<T, TT, MOIST_NOALLOC_MAX_NZ>(p, ncols, rho_w, drho_w, theta, rt2pres, dt, st);
     if (e != cudaSuccess) {
         put_msg(err, errlen, cudaGetErrorString(e));
         return MOIST_ERR_CUDA;
@@ -160,35 +226,10 @@ int moist_implicit_correction_noalloc(const moist_params* p, int precision, int 
         return MOIST_ERR_ARG;
     }
     if (ncols == 0) return MOIST_OK;
-    int dev = 0;
-    cudaError_t e = cudaGetDevice(&dev);
-    if (e != cudaSuccess || dev < 0 || dev >= kMaxDevices) {
-        put_msg(err, errlen, e != cudaSuccess ? cudaGetErrorString(e) : "device index out of range");
-        return MOIST_ERR_CUDA;
-    }
-    void* base;
-    {
-        // first call on this device: look up the scratch array's device address with the device
-        // current (the host-side symbol is only a stand-in and must never reach a kernel). The
-        // address is kept for the life of the process; it is not looked up again after a
-        // cudaDeviceReset, so no call may follow a reset of the device.
-        std::lock_guard<std::mutex> lock(g_scratch_mutex);
-        if (!g_scratch_addr[dev]) {
-            void* ptr = nullptr;
-            e = cudaGetSymbolAddress(&ptr, g_noalloc_scratch);
-            if (e != cudaSuccess || !ptr) {
-                put_msg(err, errlen, e != cudaSuccess ? cudaGetErrorString(e) : "null symbol address");
-                return MOIST_ERR_CUDA;
-            }
-            g_scratch_addr[dev] = ptr;
-        }
-        base = g_scratch_addr[dev];
-    }
     cudaStream_t st = (cudaStream_t)stream;
-    double* b = (double*)base;
-    if (precision == MOIST_F64) return run_noalloc<double, double>(p, ncols, rho_w, drho_w, theta, rt2pres, dt, st, b, err, errlen);
-    if (flags & MOIST_FLAG_TRI_NATIVE) return run_noalloc<float, float>(p, ncols, rho_w, drho_w, theta, rt2pres, dt, st, b, err, errlen);
-    return run_noalloc<float, double>(p, ncols, rho_w, drho_w, theta, rt2pres, dt, st, b, err, errlen);
+    if (precision == MOIST_F64) return run_noalloc<double, double>(p, ncols, rho_w, drho_w, theta, rt2pres, dt, st, err, errlen);
+    if (flags & MOIST_FLAG_TRI_NATIVE) return run_noalloc<float, float>(p, ncols, rho_w, drho_w, theta, rt2pres, dt, st, err, errlen);
+    return run_noalloc<float, double>(p, ncols, rho_w, drho_w, theta, rt2pres, dt, st, err, errlen);
 }
 
 #pragma GCC visibility pop
