@@ -1956,11 +1956,6 @@ __device__ __forceinline__ void b_from_ref(int nx, int nz, int halo, int P, cons
     }
 }
 template <class T>
-__global__ void k_from_ref(int nx, int nz, int halo, int P, const T* __restrict__ src, T* __restrict__ dst) {
-    b_from_ref(nx, nz, halo, P, src, dst, blockIdx.x, blockIdx.y);
-}
-
-template <class T>
 __device__ __forceinline__ void b_to_ref(int nx, int nz, int halo, int P, const T* __restrict__ src,
                                          T* __restrict__ dst, int bx, int by) {
     __shared__ T tile[32][33];
@@ -1981,26 +1976,37 @@ __device__ __forceinline__ void b_to_ref(int nx, int nz, int halo, int P, const 
         if (j < ia && k < nz) dst[(size_t)j * nz + k] = tile[threadIdx.x][r];
     }
 }
-template <class T>
-__global__ void k_to_ref(int nx, int nz, int halo, int P, const T* __restrict__ src, T* __restrict__ dst) {
-    b_to_ref(nx, nz, halo, P, src, dst, blockIdx.x, blockIdx.y);
-}
-
-// Up to 7 fields moved in one launch (blockIdx.z = field): the State's layout moves when the
-// host arrays are page-locked and mapped, so that the kernel reads or writes them over the bus
-// directly, every field's transfer in flight at once, without a staging copy.
+// The State's moves between the host layout and the device's: every 2-D field of a call in one
+// launch (blockIdx.z = field) and every 1-D one in another. Page-locked, mapped host arrays are read
+// or written over the bus directly, all fields' transfers in flight at once; a launch per field
+// cost more than the fields of a small State (733 x 77: 26 launches and 18 copies a round trip, 0.7 ms).
+constexpr int MOVE_FIELDS = 13, MOVE_ROWS = 10;
 template <class T>
 struct FieldSet {
-    const T* src[7];
-    T* dst[7];
+    const T* src[MOVE_FIELDS];
+    T* dst[MOVE_FIELDS];
+    int halo[MOVE_FIELDS];  // halo columns of the host array, 0 where only its interior is moved
 };
 template <class T>
-__global__ void k_from_ref_n(int nx, int nz, int halo, int P, FieldSet<T> f) {
-    b_from_ref(nx, nz, halo, P, f.src[blockIdx.z], f.dst[blockIdx.z], blockIdx.x, blockIdx.y);
+__global__ void k_from_ref_n(int nx, int nz, int P, FieldSet<T> f) {
+    const int j = blockIdx.z;
+    b_from_ref(nx, nz, f.halo[j], P, f.src[j], f.dst[j], blockIdx.x, blockIdx.y);
 }
 template <class T>
-__global__ void k_to_ref_n(int nx, int nz, int halo, int P, FieldSet<T> f) {
-    b_to_ref(nx, nz, halo, P, f.src[blockIdx.z], f.dst[blockIdx.z], blockIdx.x, blockIdx.y);
+__global__ void k_to_ref_n(int nx, int nz, int P, FieldSet<T> f) {
+    const int j = blockIdx.z;
+    b_to_ref(nx, nz, f.halo[j], P, f.src[j], f.dst[j], blockIdx.x, blockIdx.y);
+}
+template <class T>
+struct RowSet {
+    const T* src[MOVE_ROWS];
+    T* dst[MOVE_ROWS];
+    int n[MOVE_ROWS];
+};
+template <class T>
+__global__ void k_move_rows(RowSet<T> r) {  // blockIdx.y = array
+    const int j = blockIdx.y, i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < r.n[j]) r.dst[j][i] = r.src[j][i];
 }
 
 }  // namespace moist

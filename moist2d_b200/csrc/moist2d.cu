@@ -13,6 +13,8 @@
 #include <cstdarg>
 #include <cstdio>
 #include <cstring>
+#include <map>
+#include <mutex>
 #include <string>
 #include <thread>
 #include <vector>
@@ -121,6 +123,31 @@ int set_err(moist_ctx* c, int code, const char* fmt, ...) {
             return set_err(owner, MOIST_ERR_CUDA, "kernel launch failed: %s", cudaGetErrorString(e_));  \
     } while (0)
 
+// Properties of a device, read once per process: they do not change, and the clock rate's query alone
+// takes about a millisecond, more than the rest of a small context's creation.
+struct DeviceInfo {
+    int nsm = 0, coop = 0, optin = 0, clk_khz = 0;
+};
+cudaError_t device_info(DeviceInfo& out) {
+    static std::mutex mu;
+    static std::map<int, DeviceInfo> known;
+    int dev = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e != cudaSuccess) return e;
+    std::lock_guard<std::mutex> lock(mu);
+    auto it = known.find(dev);
+    if (it == known.end()) {
+        DeviceInfo d;
+        if ((e = cudaDeviceGetAttribute(&d.nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess) return e;
+        if ((e = cudaDeviceGetAttribute(&d.coop, cudaDevAttrCooperativeLaunch, dev)) != cudaSuccess) return e;
+        if ((e = cudaDeviceGetAttribute(&d.optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev)) != cudaSuccess) return e;
+        if ((e = cudaDeviceGetAttribute(&d.clk_khz, cudaDevAttrClockRate, dev)) != cudaSuccess) return e;
+        it = known.emplace(dev, d).first;
+    }
+    out = it->second;
+    return cudaSuccess;
+}
+
 inline unsigned cdiv(int a, int b) { return (unsigned)((a + b - 1) / b); }
 
 #define SINGLE_ARG(...) __VA_ARGS__
@@ -225,7 +252,9 @@ struct Ctx : CtxBase {
     T *halo_vals;  // [0] = rho_u[ks, is-1], [1] = rho[ks, ie+1] as of the last exchange
     T *g_dz, *g_z, *g_zf;
     double* g_trcp = nullptr;  // [nz][TEND_NRCP] reciprocals of the slow tendencies (kernels.cuh)
-    T* staging;
+    T* staging;        // stage_n host fields, stage_ld elements apart
+    int stage_n = 1;
+    size_t stage_ld = 0;
     int* err;
     CSum* bud_part;   // [BUDGET_BLOCKS][4] block sums of the budgets
     double* bud_res;  // [4]
@@ -312,8 +341,28 @@ struct Ctx : CtxBase {
         for (void* a : allocs) cudaFree(a);
     }
 
+    // The arrays of a context come from one zeroed allocation sized in init() (about 75 arrays: 75
+    // allocations, clears and frees took most of a one-shot call); what it does not hold, and what later calls
+    // add, is allocated by itself.
+    unsigned char* arena = nullptr;
+    size_t arena_left = 0;
+    int reserve(size_t bytes) {
+        if (int r = alloc(&arena, bytes)) return r;
+        CK(cudaMemsetAsync(arena, 0, bytes, st));
+        arena_left = bytes;
+        return MOIST_OK;
+    }
+    bool in_arena = false;  // the last alloc() came from the zeroed arena
+
     template <class U>
     int alloc(U** ptr, size_t n) {
+        const size_t need = (std::max<size_t>(n, 1) * sizeof(U) + 255) / 256 * 256;
+        if (in_arena = need <= arena_left; in_arena) {
+            *ptr = (U*)arena;
+            arena += need;
+            arena_left -= need;
+            return MOIST_OK;
+        }
         void* q = nullptr;
         cudaError_t e = cudaMalloc(&q, std::max<size_t>(n, 1) * sizeof(U));
         if (e != cudaSuccess) return set_err(owner, MOIST_ERR_NOMEM, "cudaMalloc of %zu bytes failed: %s", n * sizeof(U), cudaGetErrorString(e));
@@ -326,7 +375,7 @@ struct Ctx : CtxBase {
     do {                                         \
         int r_ = alloc(&(ptr), (n));             \
         if (r_ != MOIST_OK) return r_;           \
-        CK(cudaMemsetAsync((ptr), 0, std::max<size_t>((n), 1) * sizeof(*(ptr)), st)); \
+        if (!in_arena) CK(cudaMemsetAsync((ptr), 0, std::max<size_t>((n), 1) * sizeof(*(ptr)), st)); \
     } while (0)
 
     // device copies of nf whole fields (up to 8) in one launch
@@ -360,6 +409,18 @@ struct Ctx : CtxBase {
         fsz = (size_t)nz * P;
         st = owner->stream;
         dp = make_params<T>(c, P);
+        stage_ld = (host_field() + 63) / 64 * 64;
+        // pageable host fields go through staging: all 13 at a time in small contexts, fewer where 13 exceed 16 MiB
+        stage_n = (int)std::min<size_t>(MOVE_FIELDS, std::max<size_t>(1, (16u << 20) / (stage_ld * sizeof(T))));
+        // 49 fields of T, 3 of TT, 8 rows, staging, grid vectors and reciprocals, error words and budgets,
+        // the tiles' strips and words, the streaming sweep's records
+        if (int r = reserve((49 * fsz + stage_ld * stage_n + 8 * (size_t)P + 4 * (size_t)nz) * sizeof(T) + 3 * fsz * sizeof(TT) +
+                            (size_t)nz * TEND_NRCP * sizeof(double) + BUDGET_BLOCKS * 4 * sizeof(CSum) +
+                            (size_t)cdiv(nx, TT_W) * cdiv(nz, TT_H) * (TT_RING * 3 * 4 * TT_W * sizeof(T) + 64) +
+                            ((owner->flags & MOIST_FLAG_TRACER_STREAM) && nz <= STREAM_MAX_ROWS
+                                 ? skew_rows(nx, nz) * skew_pitch(nz) * (SK_ND + 3 * SK_NT) * sizeof(T) : 0) +
+                            90 * 256))
+            return r;
         for (T** f : {&cur.rho, &cur.ru, &cur.rw, &cur.rt, &cur.qv, &cur.qc, &cur.qr, &nxt.rho, &nxt.ru, &nxt.rw,
                       &nxt.rt, &nxt.qv, &nxt.qc, &nxt.qr, &tmpq[0], &tmpq[1], &tmpq[2], &ph.d_rho, &ph.d_u,
                       &ph.d_th, &ph.d_qv, &ph.d_qc, &ph.d_qr, &d_th_mp, &d_qv_mp, &d_qc_mp, &d_qr_mp, &d_qr_sed,
@@ -376,7 +437,7 @@ struct Ctx : CtxBase {
         AL(g_dz, (size_t)nz);
         AL(g_z, (size_t)nz);
         AL(g_zf, (size_t)nz);
-        AL(staging, (size_t)nz * (nx + 2 * halo) + 32);
+        AL(staging, stage_ld * stage_n);
         AL(err, 4);  // [0] halt (NaN field), [1] pending NaN field, [2] timeout, [3] spare
         AL(bud_part, (size_t)BUDGET_BLOCKS * 4);
         AL(bud_res, 4);
@@ -432,10 +493,9 @@ struct Ctx : CtxBase {
         const size_t n = skew_rows(nx, nz) * skew_pitch(nz);
         AL(skew_dom, n * SK_ND);
         for (int t = 0; t < 3; t++) AL(skew_trc[t], n * SK_NT);
-        int dev = 0, optin = 0;
-        CK(cudaGetDevice(&dev));
-        CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
-        CK(cudaFuncSetAttribute(k_tracer_stream<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
+        DeviceInfo di;
+        CK(device_info(di));
+        CK(cudaFuncSetAttribute(k_tracer_stream<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, di.optin));
         return MOIST_OK;
     }
 
@@ -447,9 +507,9 @@ struct Ctx : CtxBase {
     // Strip width: the widest of 8, 4, 2, 1 columns that still gives every SM a block and
     // keeps two blocks' shared memory on an SM; one column always fits (nz <= 1024).
     int init_strips() {
-        int dev = 0, nsm = 0;
-        CK(cudaGetDevice(&dev));
-        CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
+        DeviceInfo di;
+        CK(device_info(di));
+        const int nsm = di.nsm, optin = di.optin;
         strip_wc = 1;
         for (int w : {8, 4, 2}) {
             if (cdiv(nx, w) >= nsm && strip_smem_bytes<T, TT>(nz, w) <= 96 * 1024) {
@@ -461,8 +521,6 @@ struct Ctx : CtxBase {
         // the limit is a property of the kernel, shared by every context of the process (whose
         // strips differ, and a batch widens its members' strips): allow the device maximum, the
         // launch's own size sets the occupancy
-        int optin = 0;
-        CK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev));
         CK(cudaFuncSetAttribute(k_thomas_strip<T, TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
         CK(cudaFuncSetAttribute(k_substep_strip<T, TT>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
         rd_wc = rd_strip<T>(nx, nz, nsm);
@@ -479,10 +537,10 @@ struct Ctx : CtxBase {
         tctl.ntiles = tctl.tiles_x * tctl.tiles_z;
         tile_smem = sizeof(TileSmem<T>);
         if (owner->flags & (MOIST_FLAG_TRACER_WAVEFRONT | MOIST_FLAG_TRACER_STREAM)) return MOIST_OK;
-        int dev = 0, nsm = 0, coop = 0, nb = 0;
-        CK(cudaGetDevice(&dev));
-        CK(cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev));
-        CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+        DeviceInfo di;
+        CK(device_info(di));
+        const int nsm = di.nsm, coop = di.coop;
+        int nb = 0;
         CK(cudaFuncSetAttribute(k_tracer_tiles<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_smem));
         CK(cudaFuncSetAttribute(k_tracer_tiles<T, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)tile_smem));
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_tracer_tiles<T, false>, 96, tile_smem));
@@ -491,8 +549,10 @@ struct Ctx : CtxBase {
         const int nchunk = (tctl.tiles_x + fit - 1) / fit;
         tctl.chunk_x = (tctl.tiles_x + nchunk - 1) / nchunk;
         tctl.max_pass = tctl.chunk_x + tctl.tiles_z + 2;
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_tracer_tiles<T, true>, 96, tile_smem));
-        tiles_df_fit = nchunk == 1 && nb * nsm >= tctl.ntiles;
+        if (nchunk == 1) {
+            CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k_tracer_tiles<T, true>, 96, tile_smem));
+            tiles_df_fit = nb * nsm >= tctl.ntiles;
+        }
         // the dataflow sweep uses TT_RING versions of the strips
         AL(strips, (size_t)TT_RING * 3 * tctl.ntiles * 4 * TT_W);
         AL(tctl.ver, (size_t)3 * tctl.ntiles);
@@ -504,9 +564,7 @@ struct Ctx : CtxBase {
         tctl.pass_ts = nullptr;
         tctl.pass_work = nullptr;
         tctl.timeout = err + 2;
-        int clk = 0;
-        CK(cudaDeviceGetAttribute(&clk, cudaDevAttrClockRate, dev));  // kHz
-        tctl.spin_limit = (long long)clk * 1000LL * 2;                 // about two seconds
+        tctl.spin_limit = (long long)di.clk_khz * 1000LL * 2;  // about two seconds
         wait_default = tctl.spin_limit;
         use_tiles = true;
         tiles_df = tiles_df_fit && (owner->flags & MOIST_FLAG_TRACER_DATAFLOW) != 0;
@@ -550,96 +608,93 @@ struct Ctx : CtxBase {
         return at.type == cudaMemoryTypeHost ? at.devicePointer : nullptr;
     }
 
-    // the prognostic fields of a host State in one launch when every given array is mapped
-    // (done = false, and nothing moved, otherwise)
-    int put2d_mapped(const void* const host[7], T* const dev[7], bool& done) {
-        done = false;
-        FieldSet<T> fs{};
-        int nf = 0;
-        for (int j = 0; j < 7; j++) {
-            if (!host[j]) continue;
-            const void* hd = mapped(host[j]);
-            if (!hd) return MOIST_OK;
-            fs.src[nf] = (const T*)hd;
-            fs.dst[nf] = dev[j];
-            nf++;
-        }
-        if (nf == 0) return MOIST_OK;
-        k_from_ref_n<T><<<dim3(cdiv(nz, 32), cdiv(nx, 32), nf), dim3(32, 8), 0, st>>>(nx, nz, halo, P, fs);
-        CKL();
-        done = true;
-        return MOIST_OK;
-    }
-    int get2d_mapped(const T* const dev[7], void* const host[7], bool& done) {
-        done = false;
-        FieldSet<T> fs{};
-        int nf = 0;
-        for (int j = 0; j < 7; j++) {
-            if (!host[j]) continue;
-            void* hd = mapped(host[j]);
-            if (!hd) return MOIST_OK;
-            fs.src[nf] = dev[j];
-            fs.dst[nf] = (T*)hd;
-            nf++;
-        }
-        if (nf == 0) return MOIST_OK;
-        const int ia = nx + 2 * halo;
-        k_to_ref_n<T><<<dim3(cdiv(nz, 32), cdiv(ia, 32), nf), dim3(32, 8), 0, st>>>(nx, nz, halo, P, fs);
-        CKL();
-        done = true;
-        return MOIST_OK;
-    }
-
-    int put2d(const void* host, T* dev) {
-        if (!host) return MOIST_OK;
-        if (const void* hd = mapped(host)) {
-            dim3 b(32, 8), g(cdiv(nz, 32), cdiv(nx, 32));
-            k_from_ref<T><<<g, b, 0, st>>>(nx, nz, halo, P, (const T*)hd, dev);
-            CKL();
-            return MOIST_OK;
-        }
-        const size_t n = (size_t)nz * (nx + 2 * halo);
-        CK(cudaMemcpyAsync(staging, host, n * sizeof(T), cudaMemcpyHostToDevice, st));
-        dim3 b(32, 8), g(cdiv(nz, 32), cdiv(nx, 32));
-        k_from_ref<T><<<g, b, 0, st>>>(nx, nz, halo, P, staging, dev);
-        CKL();
-        return MOIST_OK;
-    }
-    int get2d(const T* dev, void* host, bool halos) {
-        if (!host) return MOIST_OK;
-        const int ia = nx + 2 * halo;
-        const size_t n = (size_t)nz * ia;
-        if (void* hd = mapped(host)) {  // written in place: the caller's halo columns stay as they are
-            dim3 b(32, 8), g(cdiv(nz, 32), cdiv(halos ? ia : nx, 32));
-            if (halos)
-                k_to_ref<T><<<g, b, 0, st>>>(nx, nz, halo, P, dev, (T*)hd);
+    // Moves of a call: 2-D fields in one launch per direction where the host arrays are mapped, pageable ones
+    // through staging, stage_n fields at a time; 1-D arrays in one launch, pageable ones by copies.
+    struct Moves {
+        FieldSet<T> f{};
+        RowSet<T> r{};
+        int nf = 0, nr = 0, nmax = 0;
+        int staged = 0;                                   // pageable fields in this group
+        std::array<std::pair<void*, const T*>, MOVE_FIELDS> out;  // their host arrays and staging slots (downloads)
+        std::array<size_t, MOVE_FIELDS> bytes;
+    };
+    size_t host_field() const { return (size_t)nz * (nx + 2 * halo); }
+    int flush_2d(Moves& m, bool up) {
+        if (m.nf) {
+            if (up)
+                k_from_ref_n<T><<<dim3(cdiv(nz, 32), cdiv(nx, 32), m.nf), dim3(32, 8), 0, st>>>(nx, nz, P, m.f);
             else
-                k_to_ref<T><<<g, b, 0, st>>>(nx, nz, 0, P, dev, (T*)hd + (size_t)halo * nz);
+                k_to_ref_n<T><<<dim3(cdiv(nz, 32), cdiv(nx + 2 * halo, 32), m.nf), dim3(32, 8), 0, st>>>(nx, nz, P, m.f);
             CKL();
+        }
+        for (int j = 0; j < m.staged && !up; j++)
+            CK(cudaMemcpyAsync(m.out[j].first, m.out[j].second, m.bytes[j], cudaMemcpyDeviceToHost, st));
+        m.nf = m.staged = 0;
+        return MOIST_OK;
+    }
+    int put2d(Moves& m, const void* host, T* dev) {
+        if (!host) return MOIST_OK;
+        if (m.nf == MOVE_FIELDS)
+            if (int r = flush_2d(m, true)) return r;
+        const T* src = (const T*)mapped(host);
+        if (!src) {
+            if (m.staged == stage_n)
+                if (int r = flush_2d(m, true)) return r;
+            T* slot = staging + (size_t)m.staged * stage_ld;
+            CK(cudaMemcpyAsync(slot, host, host_field() * sizeof(T), cudaMemcpyHostToDevice, st));
+            m.staged++;
+            src = slot;
+        }
+        m.f.src[m.nf] = src;
+        m.f.dst[m.nf] = dev;
+        m.f.halo[m.nf++] = halo;
+        return MOIST_OK;
+    }
+    // halos: the halo columns are written as periodic copies; otherwise the caller's stay as they are
+    int get2d(Moves& m, const T* dev, void* host, bool halos) {
+        if (!host) return MOIST_OK;
+        if (m.nf == MOVE_FIELDS)
+            if (int r = flush_2d(m, false)) return r;
+        const size_t off = halos ? 0 : (size_t)halo * nz;  // columns are contiguous
+        T* dst = (T*)mapped(host);
+        if (dst) {
+            dst += off;
+        } else {
+            if (m.staged == stage_n)
+                if (int r = flush_2d(m, false)) return r;
+            dst = staging + (size_t)m.staged * stage_ld;
+            m.out[m.staged] = {(T*)host + off, dst};
+            m.bytes[m.staged++] = (halos ? host_field() : (size_t)nz * nx) * sizeof(T);
+        }
+        m.f.src[m.nf] = dev;
+        m.f.dst[m.nf] = dst;
+        m.f.halo[m.nf++] = halos ? halo : 0;
+        return MOIST_OK;
+    }
+    // n elements between a host array (from element `at`) and a device array
+    int row(Moves& m, const void* host, int at, const T* dev, int n, bool up) {
+        if (!host) return MOIST_OK;
+        T* h = (T*)host + at;
+        T* hd = (T*)mapped(host);
+        if (!hd) {
+            if (up)
+                CK(cudaMemcpyAsync((T*)dev, h, n * sizeof(T), cudaMemcpyHostToDevice, st));
+            else
+                CK(cudaMemcpyAsync(h, dev, n * sizeof(T), cudaMemcpyDeviceToHost, st));
             return MOIST_OK;
         }
-        if (!halos) {  // keep the caller's halo columns: start from their current values
-            CK(cudaMemcpyAsync(staging, host, n * sizeof(T), cudaMemcpyHostToDevice, st));
-        }
-        dim3 b(32, 8), g(cdiv(nz, 32), cdiv(halos ? ia : nx, 32));
-        if (halos) {
-            k_to_ref<T><<<g, b, 0, st>>>(nx, nz, halo, P, dev, staging);
-        } else {
-            // interior only: write columns halo .. halo+nx-1 through an offset view
-            k_to_ref<T><<<g, b, 0, st>>>(nx, nz, 0, P, dev, staging + (size_t)halo * nz);
-        }
-        CKL();
-        CK(cudaMemcpyAsync(host, staging, n * sizeof(T), cudaMemcpyDeviceToHost, st));
+        m.r.src[m.nr] = up ? hd + at : dev;
+        m.r.dst[m.nr] = up ? (T*)dev : hd + at;
+        m.r.n[m.nr++] = n;
+        m.nmax = std::max(m.nmax, n);
         return MOIST_OK;
     }
-    int put1dx(const void* host, T* dev) {
-        if (!host) return MOIST_OK;
-        CK(cudaMemcpyAsync(dev, (const T*)host + halo, nx * sizeof(T), cudaMemcpyHostToDevice, st));
-        return MOIST_OK;
-    }
-    int get1dx(const T* dev, void* host) {
-        if (!host) return MOIST_OK;
-        CK(cudaMemcpyAsync((T*)host + halo, dev, nx * sizeof(T), cudaMemcpyDeviceToHost, st));
+    int flush(Moves& m, bool up) {
+        if (int r = flush_2d(m, up)) return r;
+        if (m.nr) {
+            k_move_rows<T><<<dim3(cdiv(m.nmax, 256), m.nr), 256, 0, st>>>(m.r);
+            CKL();
+        }
         return MOIST_OK;
     }
 
@@ -651,35 +706,29 @@ struct Ctx : CtxBase {
     }
 
     // queue the copies and layout moves of a host State on the stream (no synchronisation;
-    // stream order keeps the single staging buffer consistent)
+    // stream order keeps the staging slots consistent)
     int queue_upload(const moist_state_host* s) {
-        int r;
         StateP<T>& d = cur;
-        const void* f2[7] = {s->rho, s->rho_u, s->rho_w, s->rho_theta, s->rho_qv, s->rho_qc, s->rho_qr};
-        T* dv[7] = {d.rho, d.ru, d.rw, d.rt, d.qv, d.qc, d.qr};
-        bool done = false;
-        if ((r = put2d_mapped(f2, dv, done)) != MOIST_OK) return r;
-        for (int j = 0; j < 7 && !done; j++)
-            if ((r = put2d(f2[j], dv[j])) != MOIST_OK) return r;
-        const void* g2[6] = {s->d_rho_theta_mp, s->d_rho_qv_mp, s->d_rho_qc_mp, s->d_rho_qr_mp, s->d_rho_qr_sed,
-                             s->d_rho_theta_rd};
-        T* gv[6] = {d_th_mp, d_qv_mp, d_qc_mp, d_qr_mp, d_qr_sed, d_th_rd};
-        for (int j = 0; j < 6; j++)
-            if ((r = put2d(g2[j], gv[j])) != MOIST_OK) return r;
+        const void* f2[13] = {s->rho, s->rho_u, s->rho_w, s->rho_theta, s->rho_qv, s->rho_qc, s->rho_qr,
+                              s->d_rho_theta_mp, s->d_rho_qv_mp, s->d_rho_qc_mp, s->d_rho_qr_mp, s->d_rho_qr_sed,
+                              s->d_rho_theta_rd};
+        T* dv[13] = {d.rho, d.ru, d.rw, d.rt, d.qv, d.qc, d.qr, d_th_mp, d_qv_mp, d_qc_mp, d_qr_mp, d_qr_sed, d_th_rd};
+        Moves m;
+        for (int j = 0; j < 13; j++)
+            if (int r = put2d(m, f2[j], dv[j])) return r;
         if (s->d_rho_theta_rd) rd_dirty = true;
         sf_dirty = true;
-        const void* f1[8] = {s->prec, s->mflux, s->shflux, s->lhflux, s->d_rho_u_sf, s->d_rho_theta_sf,
-                             s->d_rho_qv_sf, nullptr};
-        T* d1[8] = {prec, mflux, shflux, lhflux, d_u_sf, d_th_sf, d_qv_sf, nullptr};
+        const void* f1[7] = {s->prec, s->mflux, s->shflux, s->lhflux, s->d_rho_u_sf, s->d_rho_theta_sf, s->d_rho_qv_sf};
+        T* d1[7] = {prec, mflux, shflux, lhflux, d_u_sf, d_th_sf, d_qv_sf};
         for (int j = 0; j < 7; j++)
-            if ((r = put1dx(f1[j], d1[j])) != MOIST_OK) return r;
-        if (s->theta_ref) CK(cudaMemcpyAsync(theta_ref, s->theta_ref, nz * sizeof(T), cudaMemcpyHostToDevice, st));
+            if (int r = row(m, f1[j], halo, d1[j], nx, true)) return r;
+        if (int r = row(m, s->theta_ref, 0, theta_ref, nz, true)) return r;
         // halo values the surface fluxes read before the next exchange (moist.jl:723, 736)
         if (halo >= 1) {
-            if (s->rho_u) CK(cudaMemcpyAsync(halo_vals, (const T*)s->rho_u + (size_t)(halo - 1) * nz, sizeof(T), cudaMemcpyHostToDevice, st));
-            if (s->rho) CK(cudaMemcpyAsync(halo_vals + 1, (const T*)s->rho + (size_t)(nx + halo) * nz, sizeof(T), cudaMemcpyHostToDevice, st));
+            if (int r = row(m, s->rho_u, (halo - 1) * nz, halo_vals, 1, true)) return r;
+            if (int r = row(m, s->rho, (nx + halo) * nz, halo_vals + 1, 1, true)) return r;
         }
-        return MOIST_OK;
+        return flush(m, true);
     }
 
     int download(moist_state_host* s) override {
@@ -690,26 +739,20 @@ struct Ctx : CtxBase {
     }
 
     int queue_download(moist_state_host* s) {
-        int r;
-        void* f2[7] = {s->rho, s->rho_u, s->rho_w, s->rho_theta, s->rho_qv, s->rho_qc, s->rho_qr};
-        const T* dv[7] = {cur.rho, cur.ru, cur.rw, cur.rt, cur.qv, cur.qc, cur.qr};
-        bool done = false;
-        if ((r = get2d_mapped(dv, f2, done)) != MOIST_OK) return r;
-        for (int j = 0; j < 7 && !done; j++) {
-            if ((r = get2d(dv[j], f2[j], true)) != MOIST_OK) return r;
-        }
-        void* g2[6] = {s->d_rho_theta_mp, s->d_rho_qv_mp, s->d_rho_qc_mp, s->d_rho_qr_mp, s->d_rho_qr_sed,
-                       s->d_rho_theta_rd};
-        T* gv[6] = {d_th_mp, d_qv_mp, d_qc_mp, d_qr_mp, d_qr_sed, d_th_rd};
-        for (int j = 0; j < 6; j++) {
-            if ((r = get2d(gv[j], g2[j], false)) != MOIST_OK) return r;
-        }
+        void* f2[13] = {s->rho, s->rho_u, s->rho_w, s->rho_theta, s->rho_qv, s->rho_qc, s->rho_qr,
+                        s->d_rho_theta_mp, s->d_rho_qv_mp, s->d_rho_qc_mp, s->d_rho_qr_mp, s->d_rho_qr_sed,
+                        s->d_rho_theta_rd};
+        const T* dv[13] = {cur.rho, cur.ru, cur.rw, cur.rt, cur.qv, cur.qc, cur.qr,
+                           d_th_mp, d_qv_mp, d_qc_mp, d_qr_mp, d_qr_sed, d_th_rd};
+        Moves m;
+        for (int j = 0; j < 13; j++)
+            if (int r = get2d(m, dv[j], f2[j], j < 7)) return r;
         void* f1[7] = {s->prec, s->mflux, s->shflux, s->lhflux, s->d_rho_u_sf, s->d_rho_theta_sf, s->d_rho_qv_sf};
-        T* d1[7] = {prec, mflux, shflux, lhflux, d_u_sf, d_th_sf, d_qv_sf};
+        const T* d1[7] = {prec, mflux, shflux, lhflux, d_u_sf, d_th_sf, d_qv_sf};
         for (int j = 0; j < 7; j++)
-            if ((r = get1dx(d1[j], f1[j])) != MOIST_OK) return r;
-        if (s->theta_ref) CK(cudaMemcpyAsync(s->theta_ref, theta_ref, nz * sizeof(T), cudaMemcpyDeviceToHost, st));
-        return MOIST_OK;
+            if (int r = row(m, f1[j], halo, d1[j], nx, false)) return r;
+        if (int r = row(m, s->theta_ref, 0, theta_ref, nz, false)) return r;
+        return flush(m, false);
     }
 
     // ------------------------------------------------------------------ the large step
@@ -1110,15 +1153,17 @@ struct Ctx : CtxBase {
         }
         const void* f2[7] = {s0->rho, s0->rho_u, s0->rho_w, s0->rho_theta, s0->rho_qv, s0->rho_qc, s0->rho_qr};
         T* dv[7] = {s0b.rho, s0b.ru, s0b.rw, s0b.rt, s0b.qv, s0b.qc, s0b.qr};
+        Moves m;
         for (int j = 0; j < 7; j++) {
             if (!f2[j]) return set_err(owner, MOIST_ERR_ARG, "s0 field %d is NULL", j);
-            if ((r = put2d(f2[j], dv[j])) != MOIST_OK) return r;
+            if ((r = put2d(m, f2[j], dv[j])) != MOIST_OK) return r;
         }
         T* pv[6] = {ph.d_rho, ph.d_u, ph.d_th, ph.d_qv, ph.d_qc, ph.d_qr};
         for (int j = 0; j < 6; j++) {
             if (!phys[j]) return set_err(owner, MOIST_ERR_ARG, "phys field %d is NULL", j);
-            if ((r = put2d(phys[j], pv[j])) != MOIST_OK) return r;
+            if ((r = put2d(m, phys[j], pv[j])) != MOIST_OK) return r;
         }
+        if ((r = flush(m, true)) != MOIST_OK) return r;
         CK(reset_err());
         T* const nq[3] = {nxt.qv, nxt.qc, nxt.qr};
         if ((r = run_stage(cur, s0b, nq, nxt, (T)dt, ns_s)) != MOIST_OK) return r;
