@@ -87,7 +87,7 @@ struct BThomas {
     T dt_s;
     int wc;
     T *ta, *tb, *tc;
-    TT *tcp, *tpiv;
+    TT *tcp, *tpiv, *trp;
     const int* err;
 };
 template <class T, class TT>
@@ -196,7 +196,8 @@ struct FSubAsync {
 template <class T, class TT>
 struct FThomasStrip {
     __device__ void operator()(const BThomas<T, TT>& a, int bx, int by) const {
-        b_thomas_strip<T, TT>(a.p, a.theta, a.rt2pres, a.dt_s, a.wc, a.ta, a.tb, a.tc, a.tcp, a.tpiv, a.err, bx, by);
+        b_thomas_strip<T, TT>(a.p, a.theta, a.rt2pres, a.dt_s, a.wc, a.ta, a.tb, a.tc, a.tcp, a.tpiv, a.trp, a.err, bx,
+                              by);
     }
 };
 template <class T, class TT>

@@ -292,19 +292,22 @@ struct IeeeDiv {
 // 1990) with an exact acceptance test in place of a proof for every operand. On B200 the
 // dependent path is 69 cycles against 112 for IEEE division (with the multiply-subtract of a
 // Thomas level in both).
-__device__ __forceinline__ double qdiv_checked(double a, double b, double y, bool& ok) {
-    const double q0 = a * y;
-    const double r0 = fma(-b, q0, a);
-    const double q1 = fma(r0, y, q0);
+__device__ __forceinline__ bool quotient_proven(double a, double b, double q1) {
     const double r1 = fma(-b, q1, a);
     const unsigned long long bits = (unsigned long long)__double_as_longlong(q1) & 0x7fffffffffffffffULL;
     const long long e = (long long)(bits >> 52);                                   // biased exponent of q1
     const long long he = e - 53 - ((bits & 0xfffffffffffffULL) == 0 ? 1 : 0);  // half of the smaller ulp
     const double half_u = __longlong_as_double((he < 1 ? 1LL : he) << 52);
     const double aa = fabs(a), ab = fabs(b);
-    const bool zero = aa == 0.0;
     const bool in_range = aa >= 0x1p-960 && aa <= 0x1p1000 && ab >= 0x1p-1000 && ab <= 0x1p1000 && he >= 1;
-    ok = ok && (zero || (in_range && fabs(r1) < ab * half_u));
+    return in_range && fabs(r1) < ab * half_u;
+}
+__device__ __forceinline__ double qdiv_checked(double a, double b, double y, bool& ok) {
+    const double q0 = a * y;
+    const double r0 = fma(-b, q0, a);
+    const double q1 = fma(r0, y, q0);
+    const bool zero = a == 0.0;
+    ok = ok && (zero || quotient_proven(a, b, q1));
     return zero ? q0 : q1;
 }
 

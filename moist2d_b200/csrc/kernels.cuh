@@ -657,7 +657,8 @@ struct SubArgs {
     T *rho_p, *rw_p, *mfx, *mfz;      // updated in place (each column owns its entries)
     const T *ta, *tb, *tc;
     const TT *tcp, *tpiv;
-    TT* dprime;                       // scratch [nz][P]
+    const TT* trp;                    // 1 / tpiv (column strips)
+    TT* dprime;                       // scratch [nz][P] (one thread per column)
 };
 
 // One acoustic substep (moist.jl:1355-1459), one thread per column i (the ensembles' form):
@@ -1255,10 +1256,13 @@ __device__ __forceinline__ void b_substep_col_async(DevParams<T> p, SubArgs<T, T
 constexpr int STRIP_THREADS = 256;
 
 // shared memory of one strip block (bytes), laid out by StripSmem
+constexpr int STRIP_LEV = 4;  // levels whose operands the eliminations read ahead
+// rows of the eliminations' arrays: the n = nz - 1 levels in whole groups, and a group to read ahead into
+__host__ __device__ inline int strip_rows(int nz) { return (nz - 1 + STRIP_LEV - 1) / STRIP_LEV * STRIP_LEV + STRIP_LEV; }
 template <class T, class TT>
 __host__ __device__ inline size_t strip_smem_bytes(int nz, int wc) {
-    const size_t n = (size_t)(nz - 1) * wc;
-    return 5 * n * sizeof(TT) + (2 * n + 2 * (size_t)nz * wc + (size_t)nz * (wc + 1)) * sizeof(T);
+    const size_t n = (size_t)strip_rows(nz) * wc;
+    return 8 * n * sizeof(TT) + (2 * (size_t)nz * wc + (size_t)nz * (wc + 1)) * sizeof(T);
 }
 
 // A loop whose iterations load from global memory and then compute, in batches: every thread
@@ -1283,6 +1287,31 @@ __device__ __forceinline__ void batched_loop(int first, int end, int stride, L l
         }
     }
 }
+// the same loop in two parts: the operands of the first batch are asked for early (preload), while
+// an earlier phase computes or waits. EARLY = false (Float64, whose batches do not fit the registers of
+// two blocks per SM: 0.42 -> 0.67 ms of substeps per step): everything in the second part.
+template <bool EARLY, class V, class L>
+__device__ __forceinline__ void batched_preload(V v[SUB_BATCH], int first, int end, int stride, L load) {
+    if constexpr (EARLY) {
+#pragma unroll
+        for (int u = 0; u < SUB_BATCH; u++) {
+            const int e = first + u * stride;
+            if (e < end) v[u] = load(e);
+        }
+    }
+}
+template <bool EARLY, class V, class L, class W>
+__device__ __forceinline__ void batched_rest(const V v[SUB_BATCH], int first, int end, int stride, L load, W work) {
+    if constexpr (EARLY) {
+#pragma unroll
+        for (int u = 0; u < SUB_BATCH; u++) {
+            const int e = first + u * stride;
+            if (e < end) work(e, v[u]);
+        }
+        first += SUB_BATCH * stride;
+    }
+    batched_loop<V>(first, end, stride, load, work);
+}
 template <class T, int N>
 struct Vals {
     T v[N];
@@ -1290,20 +1319,23 @@ struct Vals {
 
 template <class T, class TT>
 struct StripSmem {
-    TT *D, *Dp, *piv, *rp, *cp;  // [n][wc]: right-hand side, d', pivots, 1/pivots, modified super-diagonal
-    T *a, *w;                    // [n][wc]: sub-diagonal, new rho_w_p
+    TT *D, *Dp, *piv, *rp, *cp;  // [n][wc]: right-hand side, d' (d / pivot until eliminated), pivots, 1/pivots,
+                                 // modified super-diagonal
+    TT* ay;                      // [n][wc]: sub-diagonal / pivot
+    TT *a, *w;                   // [n][wc]: sub-diagonal, new rho_w_p (T values; conversions stay off the chains)
     T *rho_tp, *rt_tp;           // [nz][wc]: off-centred rho_p, rho_theta_p
     T* u;                        // [nz][wc+1]: rho_u_p at faces i0-1/2 .. i0+wc-1/2
     __device__ StripSmem(unsigned char* base, int nz, int wc) {
-        const size_t n = (size_t)(nz - 1) * wc;
+        const size_t n = (size_t)strip_rows(nz) * wc;
         D = (TT*)base;
         Dp = D + n;
         piv = Dp + n;
         rp = piv + n;
         cp = rp + n;
-        a = (T*)(cp + n);
+        ay = cp + n;
+        a = ay + n;
         w = a + n;
-        rho_tp = w + n;
+        rho_tp = (T*)(w + n);
         rt_tp = rho_tp + (size_t)nz * wc;
         u = rt_tp + (size_t)nz * wc;
     }
@@ -1313,8 +1345,8 @@ struct StripSmem {
 // recurrence per column
 template <class T, class TT>
 __device__ __forceinline__ void b_thomas_strip(DevParams<T> p, const T* theta, const T* rt2pres, T dt_s, int wc,
-                                               T* ta, T* tb, T* tc, TT* tcp, TT* tpiv, const int* err, int bx,
-                                               int by) {
+                                               T* ta, T* tb, T* tc, TT* tcp, TT* tpiv, TT* trp, const int* err,
+                                               int bx, int by) {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     if (halted(err)) return;
     const int nx = p.nx, nz = p.nz, P = p.P;
@@ -1348,7 +1380,7 @@ __device__ __forceinline__ void b_thomas_strip(DevParams<T> p, const T* theta, c
             tb[MOIST_IDX(j, i)] = b;
             tc[MOIST_IDX(j, i)] = c;
             sm.D[j * wc + col] = (TT)(b + T(1.0));
-            sm.a[j * wc + col] = a;
+            sm.a[j * wc + col] = (TT)a;
             sm.cp[j * wc + col] = (TT)c;
         });
     __syncthreads();
@@ -1356,17 +1388,17 @@ __device__ __forceinline__ void b_thomas_strip(DevParams<T> p, const T* theta, c
         // the pivot recurrence, the next level's operands read one level ahead (index clamped)
         const int cc = threadIdx.x;
         const TT* __restrict__ sD = sm.D;
-        const T* __restrict__ sa = sm.a;
+        const TT* __restrict__ sa = sm.a;
         TT* __restrict__ sc = sm.cp;
         TT* __restrict__ sp = sm.piv;
         TT cp_prev = TT(0);
-        TT bn = sD[cc], an = (TT)sa[cc], cn = sc[cc];
+        TT bn = sD[cc], an = sa[cc], cn = sc[cc];
 #pragma unroll 4
         for (int j = 0; j < n; j++) {
             const TT bb = bn, aj = an, cj = cn;
             const int jn = j + 1 < n ? j + 1 : n - 1;
             bn = sD[jn * wc + cc];
-            an = (TT)sa[jn * wc + cc];
+            an = sa[jn * wc + cc];
             cn = sc[jn * wc + cc];
             const TT piv = j == 0 ? bb : bb - aj * cp_prev;
             const TT cpj = cj / piv;
@@ -1379,12 +1411,114 @@ __device__ __forceinline__ void b_thomas_strip(DevParams<T> p, const T* theta, c
     #pragma unroll 4
     for (int j = r0; j < n && own; j += rs) {
         tcp[MOIST_IDX(j, i)] = sm.cp[j * wc + col];
-        tpiv[MOIST_IDX(j, i)] = sm.piv[j * wc + col];
+        const TT piv = sm.piv[j * wc + col];
+        tpiv[MOIST_IDX(j, i)] = piv;
+        if constexpr (sizeof(TT) == 8) trp[MOIST_IDX(j, i)] = (TT)1 / piv;  // for the substeps' quotients
     }
 }
 template <class T, class TT>
-__global__ void __launch_bounds__(STRIP_THREADS) k_thomas_strip(DevParams<T> p, const T* theta, const T* rt2pres,                                                                  T dt_s, int wc, T* ta, T* tb, T* tc, TT* tcp,                                                                  TT* tpiv, const int* err) {
-    b_thomas_strip(p, theta, rt2pres, dt_s, wc, ta, tb, tc, tcp, tpiv, err, blockIdx.x, blockIdx.y);
+__global__ void __launch_bounds__(STRIP_THREADS) k_thomas_strip(DevParams<T> p, const T* theta, const T* rt2pres,
+                                                                 T dt_s, int wc, T* ta, T* tb, T* tc, TT* tcp,
+                                                                 TT* tpiv, TT* trp, const int* err) {
+    b_thomas_strip(p, theta, rt2pres, dt_s, wc, ta, tb, tc, tcp, tpiv, trp, err, blockIdx.x, blockIdx.y);
+}
+
+// f(std::integral_constant-like width) for the strip width wc: constant offsets between the levels
+template <int W>
+struct StripWidth {
+    static constexpr int value = W;
+};
+template <class F>
+__device__ __forceinline__ void strip_by_width(int wc, F f) {
+    if (wc == 8) f(StripWidth<8>{});
+    else if (wc == 4) f(StripWidth<4>{});
+    else if (wc == 2) f(StripWidth<2>{});
+    else f(StripWidth<1>{});
+}
+// The two recurrences of column cc, STRIP_LEV levels' operands read ahead of the ones in use, without a
+// guard: the levels beyond the top are zero, the group read ahead below level 0 lies in the array before.
+template <int W, class T, class TT>
+__device__ __forceinline__ void strip_eliminate(const StripSmem<T, TT>& sm, int n, int cc) {
+    constexpr int L = STRIP_LEV;
+    const TT *sD = sm.D + cc, *sp = sm.piv + cc, *sr = sm.rp + cc, *say = sm.ay + cc;
+    const TT* sa = sm.a + cc;
+    TT* sDp = sm.Dp + cc;  // d_j y before, d'_j after
+    TT D[2][L], a[2][L], p[2][L], y[2][L], ay[2][L], dy[2][L];
+    auto load = [&](int h) {
+#pragma unroll
+        for (int u = 0; u < L; u++) {
+            D[h][u] = sD[u * W];
+            a[h][u] = sa[u * W];
+            p[h][u] = sp[u * W];
+            y[h][u] = sr[u * W];
+            ay[h][u] = say[u * W];
+        }
+        sD += L * W;
+        sa += L * W;
+        sp += L * W;
+        sr += L * W;
+        say += L * W;
+    };
+    auto load_dy = [&](int h, const TT* q) {
+#pragma unroll
+        for (int u = 0; u < L; u++) dy[h][u] = q[u * W];
+    };
+    TT dprev = (TT)0;
+    auto group = [&](int h) {
+#pragma unroll
+        for (int u = 0; u < L; u++) {
+            const TT x = D[h][u] - a[h][u] * dprev;  // a_0 = 0
+            const TT q0 = fma(-ay[h][u], dprev, dy[h][u]);
+            dprev = fma(fma(-p[h][u], q0, x), y[h][u], q0);
+            sDp[u * W] = dprev;
+        }
+        sDp += L * W;
+    };
+    load(0);
+    load_dy(0, sDp);
+    for (int j = 0; j < n; j += 2 * L) {
+        load(1);
+        load_dy(1, sDp + L * W);
+        group(0);
+        if (j + L >= n) break;
+        load(0);
+        load_dy(0, sDp + L * W);
+        group(1);
+    }
+}
+template <int W, class T, class TT>
+__device__ __forceinline__ void strip_substitute(const StripSmem<T, TT>& sm, int n, int cc) {  // x_j = d'_j - c'_j x_{j+1}
+    constexpr int L = STRIP_LEV;
+    const int top = (n + L - 1) / L * L - L;  // first level of the highest group
+    const TT *sd = sm.Dp + top * W + cc, *sc = sm.cp + top * W + cc;
+    TT* sw = sm.w + top * W + cc;
+    TT d[2][L], c[2][L];
+    auto load = [&](int h) {
+#pragma unroll
+        for (int u = 0; u < L; u++) {
+            d[h][u] = sd[u * W];
+            c[h][u] = sc[u * W];
+        }
+        sd -= L * W;
+        sc -= L * W;
+    };
+    TT x = (TT)0;
+    auto group = [&](int h) {
+#pragma unroll
+        for (int u = L - 1; u >= 0; u--) {
+            x = d[h][u] - c[h][u] * x;
+            sw[u * W] = x;
+        }
+        sw -= L * W;
+    };
+    load(0);
+    for (int j = top; j >= 0; j -= 2 * L) {
+        load(1);
+        group(0);
+        if (j - L < 0) break;
+        load(0);
+        group(1);
+    }
 }
 
 // b_substep_col over a strip (moist.jl:1355-1459)
@@ -1404,20 +1538,42 @@ __device__ __forceinline__ void b_substep_strip(DevParams<T> p, SubArgs<T, TT> a
     const T fact_tpT = T(0.5) * (T(1.0) + p.beta);
     const T fact_tmT = T(0.5) * (T(1.0) - p.beta);
     const T fact = fact_tmT / fact_tpT;
+    const int col = tid % wc, r0 = tid / wc, rs = STRIP_THREADS / wc;
+    const bool own = col < ncol;
+    const int i = i0 + col;
+    const int im = wrapx(i - 1, nx), ip = wrapx(i + 1, nx);
+    // Every phase's first operands are asked for one phase ahead: a block otherwise waits a memory round
+    // trip per phase with all its threads.
+    auto load2 = [&](int k) {
+        const size_t c = MOIST_IDX(k, i);
+        return Vals<T, 8>{{a.mfx[c], ro(a.R_rho + c), a.rho_p[c], ro(a.theta + c), ro(a.theta + MOIST_IDX(k, ip)),
+                           ro(a.theta + MOIST_IDX(k, im)), ro(a.R_rt + c), ro(a.rt_in + c)}};
+    };
+    Vals<T, 8> v2[SUB_BATCH];
+    constexpr bool EARLY = sizeof(T) == 4;
+    batched_preload<EARLY>(v2, r0, own ? nz : 0, rs, load2);
     // (1) horizontal forward step of rho_u_p at the ncol + 1 faces (1355-1366)
     {
         const int nf = ncol + 1, wf = wc + 1;
+        const float rnf = 1.0f / (float)nf;
+        // e / nf for e < 2^22: the estimate is off by one at most
+        auto row_of = [&](int e) {
+            int k = (int)((float)e * rnf);
+            if (k * nf > e) k--;
+            if ((k + 1) * nf <= e) k++;
+            return k;
+        };
         batched_loop<Vals<T, 8>>(
             tid, nz * nf, STRIP_THREADS,
             [&](int e) {
-                const int k = e / nf, f = e - k * nf;
+                const int k = row_of(e), f = e - k * nf;
                 const int cc = wrapx(i0 + f - 1, nx), cn = wrapx(cc + 1, nx);
                 const size_t a0 = MOIST_IDX(k, cc), a1 = MOIST_IDX(k, cn);
                 return Vals<T, 8>{{ro(a.rt_in + a0), ro(a.rt_in + a1), ro(a.rt_old + a0), ro(a.rt_old + a1),
                                    ro(a.rt2pres + a0), ro(a.rt2pres + a1), ro(a.ru_in + a0), ro(a.R_ru + a0)}};
             },
             [&](int e, const Vals<T, 8>& v) {
-                const int k = e / nf, f = e - k * nf;
+                const int k = row_of(e), f = e - k * nf;
                 T grad_x = (v.v[1] - v.v[0]) / dx;
                 const T grad_x_old = (v.v[3] - v.v[2]) / dx;
                 grad_x = grad_x + p.gamma_d * (grad_x - grad_x_old);
@@ -1425,19 +1581,22 @@ __device__ __forceinline__ void b_substep_strip(DevParams<T> p, SubArgs<T, TT> a
                 sm.u[k * wf + f] = v.v[6] + dt_s * (v.v[7] - rt2pres_h * grad_x);
             });
     }
+    struct RhsIn {
+        T r2j, r2k, rrw, wj, wk, ta, tb, tc;
+        TT piv, cp, rp;
+    };
+    auto load3 = [&](int j) {
+        const size_t c = MOIST_IDX(j + 1, i), cj = c - P;
+        return RhsIn{ro(a.rt2pres + cj), ro(a.rt2pres + c), ro(a.R_rw + cj), a.rw_p[cj], a.rw_p[c],
+                     ro(a.ta + cj),      ro(a.tb + cj),      ro(a.tc + cj),   ro(a.tpiv + cj), ro(a.tcp + cj),
+                     sizeof(TT) == 8 ? ro(a.trp + cj) : TT(0)};
+    };
+    RhsIn v3[SUB_BATCH];
+    batched_preload<EARLY>(v3, r0, own ? n : 0, rs, load3);
     __syncthreads();
-    const int col = tid % wc, r0 = tid / wc, rs = STRIP_THREADS / wc;
-    const bool own = col < ncol;
-    const int i = i0 + col;
-    const int im = wrapx(i - 1, nx), ip = wrapx(i + 1, nx);
     // (2) explicit rho_p, rho_theta_p and their off-centred values (1367-1396)
-    batched_loop<Vals<T, 8>>(
-        r0, own ? nz : 0, rs,
-        [&](int k) {
-            const size_t c = MOIST_IDX(k, i);
-            return Vals<T, 8>{{a.mfx[c], ro(a.R_rho + c), a.rho_p[c], ro(a.theta + c), ro(a.theta + MOIST_IDX(k, ip)),
-                               ro(a.theta + MOIST_IDX(k, im)), ro(a.R_rt + c), ro(a.rt_in + c)}};
-        },
+    batched_rest<EARLY>(
+        v2, r0, own ? nz : 0, rs, load2,
         [&](int k, const Vals<T, 8>& v) {
             const size_t c = MOIST_IDX(k, i);
             const T u_m = sm.u[k * (wc + 1) + col], u_p = sm.u[k * (wc + 1) + col + 1];
@@ -1459,17 +1618,8 @@ __device__ __forceinline__ void b_substep_strip(DevParams<T> p, SubArgs<T, TT> a
         });
     __syncthreads();
     // (3) right-hand side of the w-p system (1397-1408) and the stage factors
-    struct RhsIn {
-        T r2j, r2k, rrw, wj, wk, ta, tb, tc;
-        TT piv, cp;
-    };
-    batched_loop<RhsIn>(
-        r0, own ? n : 0, rs,
-        [&](int j) {
-            const size_t c = MOIST_IDX(j + 1, i), cj = c - P;
-            return RhsIn{ro(a.rt2pres + cj), ro(a.rt2pres + c), ro(a.R_rw + cj), a.rw_p[cj], a.rw_p[c],
-                         ro(a.ta + cj),      ro(a.tb + cj),      ro(a.tc + cj),   ro(a.tpiv + cj), ro(a.tcp + cj)};
-        },
+    batched_rest<EARLY>(
+        v3, r0, own ? n : 0, rs, load3,
         [&](int j, const RhsIn& v) {
             const int k = j + 1;
             const T buoyancy = (sm.rt_tp[k * wc + col] - sm.rt_tp[j * wc + col]) / (z[k] - z[j]);
@@ -1483,72 +1633,75 @@ __device__ __forceinline__ void b_substep_strip(DevParams<T> p, SubArgs<T, TT> a
             d -= v.tb * fact * w_j;
             if (j < n - 1) d -= v.tc * fact * v.wk;
             sm.D[j * wc + col] = (TT)d;
-            sm.a[j * wc + col] = aj;
+            sm.a[j * wc + col] = (TT)aj;
             sm.piv[j * wc + col] = v.piv;
-            if constexpr (sizeof(TT) == 8) sm.rp[j * wc + col] = (TT)1 / v.piv;  // for the checked quotients of (4)
-            sm.cp[j * wc + col] = v.cp;
+            if constexpr (sizeof(TT) == 8) {
+                sm.rp[j * wc + col] = v.rp;
+                sm.ay[j * wc + col] = (TT)aj * v.rp;
+                sm.Dp[j * wc + col] = (TT)d * v.rp;
+            }
+            sm.cp[j * wc + col] = j < n - 1 ? v.cp : TT(0);  // x_{n-1} = d'_{n-1}
         });
-    __syncthreads();
-    // (4) Thomas elimination per column (moist.jl:956-970). The loops read the next level's
-    // operands one level ahead (clamped at the ends), unrolled so that the loads leave the
-    // dependent path.
-    if (tid < ncol) {
-        const int cc = tid;
-        const TT* __restrict__ sD = sm.D;
-        const T* __restrict__ sa = sm.a;
-        const TT* __restrict__ sp = sm.piv;
-        TT* __restrict__ sDp = sm.Dp;
-        TT dprev = (TT)0;
-        bool ok = sizeof(TT) == 8;
-        if constexpr (sizeof(TT) == 8) {
-            // d'_j = (d_j - a_j d'_{j-1}) / piv_j with each quotient formed from 1/piv_j (divided in
-            // (3) by all threads) and checked exact (qdiv_checked, fastdiv.cuh): 68 instead of 171
-            // cycles per level. A column with any unproven quotient is eliminated again with IEEE
-            // division below (the right-hand sides stay in D).
-            const TT* __restrict__ sr = sm.rp;
-            dprev = qdiv_checked(sD[cc], sp[cc], sr[cc], ok);
-            sDp[cc] = dprev;
-            const int j1 = n > 1 ? 1 : 0;
-            TT dn = sD[j1 * wc + cc], an = (TT)sa[j1 * wc + cc], pn = sp[j1 * wc + cc], yn = sr[j1 * wc + cc];
-#pragma unroll 4
-            for (int j = 1; j < n; j++) {
-                const TT dj = dn, aj = an, pj = pn, yj = yn;
-                const int jn = j + 1 < n ? j + 1 : n - 1;
-                dn = sD[jn * wc + cc];
-                an = (TT)sa[jn * wc + cc];
-                pn = sp[jn * wc + cc];
-                yn = sr[jn * wc + cc];
-                dprev = qdiv_checked(dj - aj * dprev, pj, yj, ok);
-                sDp[j * wc + cc] = dprev;
-            }
-        }
-        if (!ok) {
-            dprev = sD[cc] / sp[cc];
-            sDp[cc] = dprev;
-            for (int j = 1; j < n; j++) {
-                const TT dp = (sD[j * wc + cc] - (TT)sa[j * wc + cc] * dprev) / sp[j * wc + cc];
-                sDp[j * wc + cc] = dp;
-                dprev = dp;
-            }
-        }
-        // back substitution x_j = d'_j - c'_j x_{j+1}: 43 instead of 64 cycles per level
-        const TT* __restrict__ sc = sm.cp;
-        T* __restrict__ sw = sm.w;
-        TT x = dprev;
-        sw[(n - 1) * wc + cc] = (T)x;
-        const int jb = n >= 2 ? n - 2 : 0;
-        TT dpn = sDp[jb * wc + cc], cpn = sc[jb * wc + cc];
-#pragma unroll 4
-        for (int j = n - 2; j >= 0; j--) {
-            const TT dpj = dpn, cpj = cpn;
-            const int jn = j >= 1 ? j - 1 : 0;
-            dpn = sDp[jn * wc + cc];
-            cpn = sc[jn * wc + cc];
-            x = dpj - cpj * x;
-            sw[j * wc + cc] = (T)x;
-        }
+    for (int e = n * wc + tid; e < strip_rows(nz) * wc; e += STRIP_THREADS) {  // levels beyond the top: all values stay zero
+        sm.D[e] = sm.Dp[e] = sm.ay[e] = sm.cp[e] = TT(0);
+        sm.piv[e] = sm.rp[e] = TT(1);
+        sm.a[e] = TT(0);
     }
     __syncthreads();
+    // (4) Thomas elimination per column (moist.jl:956-970), one lane per column: the chain of the kernel.
+    // Up: d'_j = (d_j - a_j d'_{j-1}) / piv_j. With y = RN(1/piv_j) (formed once per stage), a_j y and d_j y
+    // the quotient is estimated from d'_{j-1} in one FMA, while the numerator is formed in two, and
+    // corrected by its remainder: 32 cycles of dependent FP64 per level against 40 from the numerator
+    // alone (and 171 with IEEE division). The estimate is exact but for rare cases; whether every
+    // quotient is RN(x / piv) is checked by the other warps (quotient_proven) while the first one
+    // substitutes back, and a block with an unproven quotient repeats both with IEEE division.
+    auto back_substitute = [&](int cc) {
+        strip_by_width(wc, [&](auto w) { strip_substitute<decltype(w)::value>(sm, n, cc); });
+    };
+    auto eliminate_ieee = [&](int cc) {
+        TT dprev = sm.D[cc] / sm.piv[cc];
+        sm.Dp[cc] = dprev;
+        for (int j = 1; j < n; j++) {
+            dprev = (sm.D[j * wc + cc] - sm.a[j * wc + cc] * dprev) / sm.piv[j * wc + cc];
+            sm.Dp[j * wc + cc] = dprev;
+        }
+        for (int j = n; j < strip_rows(nz); j++) sm.Dp[j * wc + cc] = TT(0);  // after a non-finite first try
+    };
+    // the vertical updates' lines into L1 while the elimination runs
+    for (int k = r0; k < nz && own; k += rs) {
+        const size_t c = MOIST_IDX(k, i);
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(a.rho_p + c));
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(a.rt_out + c));
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(a.mfz + c));
+        asm volatile("prefetch.global.L1 [%0];" ::"l"(a.s_rw + c));
+    }
+    if constexpr (sizeof(TT) == 8) {
+        if (tid < ncol) strip_by_width(wc, [&](auto w) { strip_eliminate<decltype(w)::value>(sm, n, tid); });
+        __syncthreads();
+        bool unproven = false;
+        if (tid < 32) {
+            if (tid < ncol) back_substitute(tid);
+        } else {
+            for (int e = tid - 32; e < n * wc; e += STRIP_THREADS - 32) {
+                if (e % wc >= ncol) continue;
+                const TT x = e < wc ? sm.D[e] : sm.D[e] - sm.a[e] * sm.Dp[e - wc];
+                unproven |= x == TT(0) ? !same_bits(sm.Dp[e], x * sm.rp[e]) : !quotient_proven(x, sm.piv[e], sm.Dp[e]);
+            }
+        }
+        if (__syncthreads_or(unproven)) {
+            if (tid < ncol) {
+                eliminate_ieee(tid);
+                back_substitute(tid);
+            }
+            __syncthreads();
+        }
+    } else {
+        if (tid < ncol) {
+            eliminate_ieee(tid);
+            back_substitute(tid);
+        }
+        __syncthreads();
+    }
     // (5) vertical rho_p, rho_theta_p updates (1412-1446), momentum flux averages (1452-1458)
     // every value a branch may read is loaded, in bounds, before the branches select
     const T* th = a.theta;
@@ -1564,8 +1717,8 @@ __device__ __forceinline__ void b_substep_strip(DevParams<T> p, SubArgs<T, TT> a
         [&](int k, const Vals<T, 10>& v) {
             const size_t c = MOIST_IDX(k, i);
             const T th_m2 = v.v[5], th_m1 = v.v[6], th_0 = v.v[7], th_p1 = v.v[8], th_p2 = v.v[9];
-            const T w_k = k < ke ? sm.w[k * wc + col] : T(0.0);
-            const T w_km = k > 0 ? sm.w[(k - 1) * wc + col] : T(0.0);
+            const T w_k = k < ke ? (T)sm.w[k * wc + col] : T(0.0);
+            const T w_km = k > 0 ? (T)sm.w[(k - 1) * wc + col] : T(0.0);
             if (k < ke) a.rw_p[c] = w_k;
             {
                 const T flux_kp = k == ke ? T(0.0) : w_k;
@@ -1603,7 +1756,7 @@ __device__ __forceinline__ void b_substep_strip(DevParams<T> p, SubArgs<T, TT> a
         });
 }
 template <class T, class TT>
-__global__ void __launch_bounds__(STRIP_THREADS) k_substep_strip(DevParams<T> p, SubArgs<T, TT> a, T dt_s, T ns_T,                                                                   double fact_tp64, int wc, const int* err) {
+__global__ void __launch_bounds__(STRIP_THREADS, 2) k_substep_strip(DevParams<T> p, SubArgs<T, TT> a, T dt_s, T ns_T,                                                                   double fact_tp64, int wc, const int* err) {
     b_substep_strip(p, a, dt_s, ns_T, fact_tp64, wc, err, blockIdx.x, blockIdx.y);
 }
 

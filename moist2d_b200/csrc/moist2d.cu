@@ -247,7 +247,7 @@ struct Ctx : CtxBase {
     T *d_th_mp, *d_qv_mp, *d_qc_mp, *d_qr_mp, *d_qr_sed, *d_th_rd;
     T *pres, *theta, *rt2p, *uface, *wface, *R_rho, *R_ru, *R_rw, *R_rt;
     T *rho_p, *ru_p[2], *rw_p, *rt_p[3], *mfx, *mfz, *ta, *tb, *tc;
-    TT *tcp, *tpiv, *dprime;
+    TT *tcp, *tpiv, *trp, *dprime;
     T *prec, *d_prec, *mflux, *shflux, *lhflux, *d_u_sf, *d_th_sf, *d_qv_sf, *theta_ref;
     T *halo_vals;  // [0] = rho_u[ks, is-1], [1] = rho[ks, ie+1] as of the last exchange
     T *g_dz, *g_z, *g_zf;
@@ -412,9 +412,9 @@ struct Ctx : CtxBase {
         stage_ld = (host_field() + 63) / 64 * 64;
         // pageable host fields go through staging: all 13 at a time in small contexts, fewer where 13 exceed 16 MiB
         stage_n = (int)std::min<size_t>(MOVE_FIELDS, std::max<size_t>(1, (16u << 20) / (stage_ld * sizeof(T))));
-        // 49 fields of T, 3 of TT, 8 rows, staging, grid vectors and reciprocals, error words and budgets,
+        // 49 fields of T, 4 of TT, 8 rows, staging, grid vectors and reciprocals, error words and budgets,
         // the tiles' strips and words, the streaming sweep's records
-        if (int r = reserve((49 * fsz + stage_ld * stage_n + 8 * (size_t)P + 4 * (size_t)nz) * sizeof(T) + 3 * fsz * sizeof(TT) +
+        if (int r = reserve((49 * fsz + stage_ld * stage_n + 8 * (size_t)P + 4 * (size_t)nz) * sizeof(T) + 4 * fsz * sizeof(TT) +
                             (size_t)nz * TEND_NRCP * sizeof(double) + BUDGET_BLOCKS * 4 * sizeof(CSum) +
                             (size_t)cdiv(nx, TT_W) * cdiv(nz, TT_H) * (TT_RING * 3 * 4 * TT_W * sizeof(T) + 64) +
                             ((owner->flags & MOIST_FLAG_TRACER_STREAM) && nz <= STREAM_MAX_ROWS
@@ -430,6 +430,7 @@ struct Ctx : CtxBase {
         s0b = StateP<T>{nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
         AL(tcp, fsz);
         AL(tpiv, fsz);
+        AL(trp, fsz);
         AL(dprime, fsz);
         for (T** f : {&prec, &d_prec, &mflux, &shflux, &lhflux, &d_u_sf, &d_th_sf, &d_qv_sf}) AL(*f, (size_t)P);
         AL(theta_ref, (size_t)nz);
@@ -824,14 +825,14 @@ struct Ctx : CtxBase {
         if (rec) {
             rec->put(BK_DIAG, BDiag<T>{dp, s_in, pres, theta, rt2p, uface, wface, err});
             rec->put(BK_TEND, BTend<T>{dp, ta_, err});
-            rec->put(BK_THOMAS, BThomas<T, TT>{dp, theta, rt2p, dt_s, strip_wc, ta, tb, tc, tcp, tpiv, err});
+            rec->put(BK_THOMAS, BThomas<T, TT>{dp, theta, rt2p, dt_s, strip_wc, ta, tb, tc, tcp, tpiv, trp, err});
         } else {
             k_diag<T><<<g2, b2, 0, st>>>(dp, s_in, pres, theta, rt2p, uface, wface, err);
             CKL();
             k_tend<T><<<g2, b2, 0, st>>>(dp, ta_, err);
             CKL();
             k_thomas_strip<T, TT><<<gs, STRIP_THREADS, strip_smem, st>>>(dp, theta, rt2p, dt_s, strip_wc, ta, tb, tc,
-                                                                         tcp, tpiv, err);
+                                                                         tcp, tpiv, trp, err);
             CKL();
         }
         if (tape) {
@@ -865,6 +866,7 @@ struct Ctx : CtxBase {
             sa.tc = tc;
             sa.tcp = tcp;
             sa.tpiv = tpiv;
+            sa.trp = trp;
             sa.dprime = dprime;
             if (rec) {
                 rec->put(BK_SUB, BSub<T, TT>{dp, sa, dt_s, T(ns_s), fact_tp64, strip_wc, err});

@@ -2,8 +2,8 @@
 the tiled tracer sweep in chunks of tile columns (more tiles than fit on the GPU), both sweeps on
 mixing ratios that fall through the subnormal range (exact ties of the divisions included) and on a
 grid outside the range of the fast division (every tile and sweep repeated with IEEE division); the
-radiation and the column solve at every strip width, on the last partial strip, and the column
-solve's repeat with IEEE division."""
+substep, radiation and column solve at every strip width, on the last partial strip, and the column
+solve's and the substep's repeat with IEEE division."""
 import numpy as np
 import pytest
 
@@ -55,6 +55,27 @@ def test_grid_outside_the_fast_divisions_range(T, dx, flags):
     p, s = small_case(T, 45, 21, Lx=45 * dx)
     assert float(p.dx) > (2.0 ** 40 if T is np.float32 else 2.0 ** 100)
     _both(p, s, flags)
+
+
+@pytest.mark.parametrize("T,flags", [(np.float32, 0), (np.float32, abi.MOIST_FLAG_TRI_NATIVE), (np.float64, 0)],
+                         ids=["f32-tri64", "f32-tri32", "f64"])
+@pytest.mark.parametrize("nx,nz", [(299, 3), (601, 6), (1187, 9), (1187, 2), (1190, 66)])
+def test_substep_strips(T, flags, nx, nz):
+    p, s = small_case(T, nx, nz)
+    _both(p, s, flags, tri64=not flags)
+
+
+def test_substep_quotients_below_the_checked_range():
+    """Numerators of 1e-295 are refused by the exactness check: the block repeats with IEEE division."""
+    p, s = small_case(np.float64, 37, 21)
+    s.rho_w[:] = 0.0
+    z = [np.zeros((p.ka, p.ia), order="F") for _ in range(6)]
+    a, b = s.copy(), s.copy()
+    model.compute_step(z, a, s, p, 3e-295, 2)
+    bind.compute_step(z, b, s, p, 3e-295, 2)
+    w = np.abs(b.rho_w[:, p.is_ - 1:p.ie])
+    assert 0.0 < np.max(w) < 1e-290
+    compare(a, b, p)
 
 
 @pytest.mark.parametrize("T", [np.float32, np.float64])
