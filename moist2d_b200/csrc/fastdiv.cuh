@@ -240,6 +240,12 @@ struct FastDiv : DivRange<T> {
     }
     // a / b with y = prep1(b)
     __device__ __forceinline__ static T quot(T a, T b, T y, bool& bad) { return twice(a, b, y, b * DR::TIE, bad); }
+    // a / b for a variable b > 0; a result that is not finite sets bad
+    __device__ __forceinline__ static T quot_var(T a, T b, bool& bad) {
+        const T q = twice(a, b, rcp_rn(b, bad), b * DR::TIE, bad);
+        bad |= b > DR::BIG || !(fabs(q) <= DR::MAX);
+        return q;
+    }
     // the limiter ratio: |b| < EPS ? 1 : a / b (the sign of a zero is not kept for b < 0: the limiter
     // takes both zeros to +0)
     __device__ __forceinline__ static T ratio(T a, T b, T EPS, bool& bad) {
@@ -271,6 +277,7 @@ template <class T>
 struct IeeeDiv {
     __device__ __forceinline__ static T cdiv(T a, T b, const Rcp<T>&) { return a / b; }
     __device__ __forceinline__ static T quot(T a, T b, T, bool&) { return a / b; }
+    __device__ __forceinline__ static T quot_var(T a, T b, bool&) { return a / b; }
     __device__ __forceinline__ static T ratio(T a, T b, T EPS, bool&) { return fabs(b) < EPS ? T(1) : a / b; }
     __device__ __forceinline__ static T div3(T a) { return a / T(3); }
 };

@@ -418,7 +418,7 @@ struct Ctx : CtxBase {
                             (size_t)nz * TEND_NRCP * sizeof(double) + BUDGET_BLOCKS * 4 * sizeof(CSum) +
                             (size_t)cdiv(nx, TT_W) * cdiv(nz, TT_H) * (TT_RING * 3 * 4 * TT_W * sizeof(T) + 64) +
                             ((owner->flags & MOIST_FLAG_TRACER_STREAM) && nz <= STREAM_MAX_ROWS
-                                 ? skew_rows(nx, nz) * skew_pitch(nz) * (SK_ND + 3 * SK_NT) * sizeof(T) : 0) +
+                                 ? skew_elems(nx, nz) * (SK_ND + 3 * SK_NT) * sizeof(T) : 0) +
                             90 * 256))
             return r;
         for (T** f : {&cur.rho, &cur.ru, &cur.rw, &cur.rt, &cur.qv, &cur.qc, &cur.qr, &nxt.rho, &nxt.ru, &nxt.rw,
@@ -491,7 +491,7 @@ struct Ctx : CtxBase {
 
     // the records of the streaming sweep (zero where no cell writes them)
     int alloc_stream() {
-        const size_t n = skew_rows(nx, nz) * skew_pitch(nz);
+        const size_t n = skew_elems(nx, nz);
         AL(skew_dom, n * SK_ND);
         for (int t = 0; t < 3; t++) AL(skew_trc[t], n * SK_NT);
         DeviceInfo di;
@@ -584,7 +584,7 @@ struct Ctx : CtxBase {
             if (tctl.bar) CK(cudaMemsetAsync(tctl.bar, 0, 3 * sizeof(*tctl.bar), st));
             CK(reset_err());
             CK(cudaStreamSynchronize(st));
-            return set_err(owner, MOIST_ERR_TIMEOUT, "a grid barrier of the tiled tracer sweep timed out");
+            return set_err(owner, MOIST_ERR_TIMEOUT, "a bounded wait of the tracer sweep timed out");
         }
         if (h[0] != INT_MAX) {
             owner->nan_field = h[0];
@@ -2932,6 +2932,9 @@ struct BatchImpl : BatchBase {
         BCK(cudaGetLastError());
         owner->nan_member = -1;
         owner->nan_field = -1;
+        for (int i = 0; i < n; i++)
+            if (h[4 * i + 2] != 0)
+                return set_berr(owner, MOIST_ERR_TIMEOUT, "member %d: a bounded wait of the tracer sweep timed out", i);
         for (int i = 0; i < n; i++) {
             if (h[4 * i] != INT_MAX) {
                 static const char* names[12] = {"rho", "rho_u", "rho_w", "rho_theta", "rho_qv", "rho_qc", "rho_qr",

@@ -3,18 +3,21 @@
 //
 // Cell (k, i) of the in-place sweep (moist.jl:1469-1518) reads the updated values at (k, i-1),
 // (k, i-2), (k-1, i), (k-2, i) and stage-start values elsewhere, so the anti-diagonals
-// k + i = const can be updated together. One block sweeps one tracer of one domain: two lanes own
-// row k (tracer_cell.cuh; 16 rows per warp, nz <= STREAM_MAX_ROWS) and update column c = s - k at
-// step s, for s = 0 .. nx + nz - 2. No speculation, no repair passes and no grid-wide barrier:
+// k + i = const can be updated together. One block sweeps one tracer of one domain: warp g owns rows
+// 16 g .. 16 g + 15 (two lanes a row, tracer_cell.cuh; nz <= STREAM_MAX_ROWS), row 16 g + r at column
+// j - r in its step j = 0 .. nx + 14. No speculation, no repair passes and no grid-wide barrier:
 // blocks are independent, so any number of (domain, tracer) sweeps can share one launch.
 //
-// The stage-start inputs are first copied by b_stream_prep into records by anti-diagonal (element
-// k of record s belongs to column s - k), so that a step reads whole lines: with the fields' own
-// layout every lane of a load touches another row, 32 lines a load, which bounded the sweep (2900
-// cycles a step with two or three blocks of 128 rows on an SM). The block copies one record a step with
-// 16-byte cp.async into a ring of shared memory, three steps before its first use. The updated
-// values of the rows below come through warp shuffles, across warps through a small ring, one
-// block barrier per step.
+// The stage-start inputs are first copied by b_stream_prep into records by row group and
+// anti-diagonal (the element of row k in record s belongs to column s - k), so that a step reads
+// whole lines: with the fields' own layout every lane of a load touches another row, 32 lines a
+// load, which bounded the sweep. A warp copies its own records with 16-byte cp.async into its own
+// ring of shared memory, four steps ahead. It depends on the warp below alone, through the updated
+// values of that warp's two top rows: they pass through a ring of shared memory, with counts of the
+// columns done and used, read and written every STREAM_HAND steps. (With one block barrier a step,
+// and a whole block copying each record, a step took 2500 cycles, of which the cell takes about 500: the
+// slowest warp, and the copies' and the barrier's instructions, for every warp.) Waits on a count
+// are bounded and report through the error words.
 #pragma once
 
 #include "tracer_tiles.cuh"
@@ -22,22 +25,24 @@
 namespace moist {
 
 constexpr int STREAM_MAX_ROWS = 256;  // rows per block (two threads each)
-constexpr int STREAM_RING = 8;        // records in shared memory; columns kept of the two top rows of every warp
+constexpr int STREAM_RING = 8;        // records of a warp in shared memory
+constexpr int STREAM_HAND = 8;        // steps between two exchanges of counts with the neighbouring warps
+constexpr int STREAM_TOP = 64;        // columns of a warp's top rows kept for the warp above
+constexpr int SK_ROWS = 20;           // rows 16 g - 1 .. 16 g + 17 of a group at positions 0 .. 18
 
 // fields of a record: the first six are the domain's, the last three the tracer's
 enum { SK_VX = 0, SK_VZ, SK_RX, SK_RZ, SK_RHO, SK_RRHO, SK_ND, SK_S = 0, SK_Q0, SK_DPH, SK_NT };
 
-// elements of one field of a record: rows -1 .. nz+1 at positions 0 .. nz+2, padded to 16 (mod 32) so that
-// the two halves of a warp read two neighbouring fields on different banks
-__host__ __device__ inline int skew_pitch(int nz) { return (nz + 3 + 15) / 32 * 32 + 16; }
-// records s = -1 .. nx + nz + 1 (+ the ring's look-ahead)
-__host__ __device__ inline size_t skew_rows(int nx, int nz) { return (size_t)nx + nz + 4 + STREAM_RING; }
+__host__ __device__ inline int stream_groups(int nz) { return (nz + WROWS - 1) / WROWS; }
+// records of a group: anti-diagonals 16 g - 1 .. 16 g + nx + 17 and the ring's look-ahead
+__host__ __device__ inline int skew_records(int nx) { return nx + 19 + STREAM_RING + 2; }
+__host__ __device__ inline size_t skew_elems(int nx, int nz) { return (size_t)stream_groups(nz) * skew_records(nx) * SK_ROWS; }
 
 template <class T>
 struct StreamArgs {
     TracerArgs<T> tr;
-    T* dom;      // [skew_rows][SK_ND][pitch]
-    T* trc[3];   // [skew_rows][SK_NT][pitch]
+    T* dom;      // [group][record][SK_ND][SK_ROWS]
+    T* trc[3];   // [group][record][SK_NT][SK_ROWS]
 };
 
 __device__ __forceinline__ int pmod(int c, int n) {
@@ -46,44 +51,78 @@ __device__ __forceinline__ int pmod(int c, int n) {
 }
 
 // The records of the sweep: block (bx, by) takes columns 32 bx - 1 .. 32 bx + 30 of rows 32 by ..
-// 32 by + 31 (256 threads), reads every field by rows and writes it by anti-diagonals through a
-// shared tile. s = rho_q / rho (IEEE), the reciprocal of rho for quot(), face densities. Positions no
-// cell of the domain has (rows -1, nz, nz+1; corners) keep the zeros of the allocation.
+// 32 by + 31 (256 threads), reads every field by rows and writes it by anti-diagonals through
+// shared tiles, SK_BATCH fields between two barriers. s = rho_q / rho (IEEE), the reciprocal of rho for
+// quot(), face densities. A group also holds its neighbours' rows that its cells read: s of the
+// two rows above, the vertical fluxes and densities of the row below. Positions no cell of the domain has
+// (rows -1, nz, nz+1; corners) keep the zeros of the allocation.
+constexpr int SK_BATCH = 3;
 template <class T>
 __device__ __forceinline__ void b_stream_prep(DevParams<T> p, StreamArgs<T> a, const int* err, int bx, int by) {
-    __shared__ T tile[32][34];  // stride 34: a column of an anti-diagonal touches every bank once
+    __shared__ T tile[SK_BATCH][32][34];  // stride 34: a column of an anti-diagonal touches every bank once
     if (halted(err)) return;  // the same for every thread of the launch
-    const int nx = p.nx, nz = p.nz, P = p.P, np = skew_pitch(nz);
-    const int lane = threadIdx.x & 31, wid = (threadIdx.x + threadIdx.y * blockDim.x) >> 5, nw = (blockDim.x * blockDim.y) >> 5;
+    const int nx = p.nx, nz = p.nz, P = p.P, nrec = skew_records(nx);
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nw = blockDim.x >> 5;
     const int c0 = 32 * bx - 1, k0 = 32 * by;
-    // one field: val(k, i) at the periodic column i of cells (k, c) with c in [c_lo, c_hi]
-    auto field = [&](T* out, int nf, int f, int c_lo, int c_hi, int rows, auto val) {
+    struct Field {
+        T* out;
+        int nf, f, c_lo, c_hi, rows, up, dn;  // up / dn: rows of the group above / below that the record repeats
+    };
+    // fields f[0 .. SK_BATCH): val(q, k, i) at the periodic column i of cells (k, c), c in [c_lo, c_hi], k < rows
+    auto fields = [&](const Field (&f)[SK_BATCH], auto val) {
         for (int r = wid; r < 32; r += nw) {
-            const int k = k0 + r, c = c0 + lane;
-            tile[r][lane] = (k < rows && c >= c_lo && c <= c_hi) ? val(k, pmod(c, nx)) : T(0);
+            const int k = k0 + r, c = c0 + lane, i = pmod(c, nx);
+#pragma unroll
+            for (int q = 0; q < SK_BATCH; q++)
+                tile[q][r][lane] = (k < f[q].rows && c >= f[q].c_lo && c <= f[q].c_hi) ? val(q, k, i) : T(0);
         }
         __syncthreads();
-        for (int d = wid; d < 63; d += nw) {  // anti-diagonal d of the tile: rows r with column d - r
-            const int cc = d - lane, k = k0 + lane, c = c0 + cc;
-            if (cc >= 0 && cc < 32 && k < rows && c >= c_lo && c <= c_hi)
-                out[((size_t)(c + k + 1) * nf + f) * np + k + 1] = tile[lane][cc];
+        const int k = k0 + lane, g = k / WROWS, r = k - g * WROWS;
+        for (int d = wid; d < 63; d += nw) {  // anti-diagonal d of the tile: rows with column d - row
+            const int cc = d - lane, c = c0 + cc, s = c + k;
+            if (cc < 0 || cc >= 32) continue;
+#pragma unroll
+            for (int q = 0; q < SK_BATCH; q++) {
+                if (!(k < f[q].rows && c >= f[q].c_lo && c <= f[q].c_hi)) continue;
+                const T v = tile[q][lane][cc];
+                auto put = [&](int gg) {  // into group gg's record of anti-diagonal s
+                    f[q].out[(((size_t)gg * nrec + (s - WROWS * gg + 1)) * f[q].nf + f[q].f) * SK_ROWS + k - WROWS * gg + 1] = v;
+                };
+                put(g);
+                if (r < f[q].up && g > 0) put(g - 1);
+                if (r >= WROWS - f[q].dn && WROWS * (g + 1) < nz) put(g + 1);
+            }
         }
         __syncthreads();
     };
     const T* rho = a.tr.rho;
-    field(a.dom, SK_ND, SK_VX, -1, nx - 1, nz, [&](int k, int i) { return a.tr.mfx[MOIST_IDX(k, i)]; });
-    field(a.dom, SK_ND, SK_VZ, 0, nx - 1, nz - 1, [&](int k, int i) { return a.tr.mfz[MOIST_IDX(k, i)]; });
-    field(a.dom, SK_ND, SK_RX, -1, nx - 1, nz,
-          [&](int k, int i) { return (rho[MOIST_IDX(k, wrapx(i + 1, nx))] + rho[MOIST_IDX(k, i)]) * T(0.5); });
-    field(a.dom, SK_ND, SK_RZ, 0, nx - 1, nz - 1,
-          [&](int k, int i) { return f2h(rho[MOIST_IDX(k + 1, i)], rho[MOIST_IDX(k, i)], p.dz[k + 1], p.dz[k]); });
-    field(a.dom, SK_ND, SK_RHO, 0, nx - 1, nz, [&](int k, int i) { return rho[MOIST_IDX(k, i)]; });
-    field(a.dom, SK_ND, SK_RRHO, 0, nx - 1, nz, [&](int k, int i) { return FastDiv<T>::prep1(rho[MOIST_IDX(k, i)]); });
+    {
+        const Field f[SK_BATCH] = {{a.dom, SK_ND, SK_VX, -1, nx - 1, nz, 0, 0},
+                                   {a.dom, SK_ND, SK_VZ, 0, nx - 1, nz - 1, 0, 1},
+                                   {a.dom, SK_ND, SK_RX, -1, nx - 1, nz, 0, 0}};
+        fields(f, [&](int q, int k, int i) {
+            const size_t c = MOIST_IDX(k, i);
+            return q == 0 ? a.tr.mfx[c]
+                          : q == 1 ? a.tr.mfz[c] : (rho[MOIST_IDX(k, wrapx(i + 1, nx))] + rho[c]) * T(0.5);
+        });
+    }
+    {
+        const Field f[SK_BATCH] = {{a.dom, SK_ND, SK_RZ, 0, nx - 1, nz - 1, 0, 1},
+                                   {a.dom, SK_ND, SK_RHO, 0, nx - 1, nz, 0, 0},
+                                   {a.dom, SK_ND, SK_RRHO, 0, nx - 1, nz, 0, 0}};
+        fields(f, [&](int q, int k, int i) {
+            const size_t c = MOIST_IDX(k, i);
+            return q == 0 ? f2h(rho[c + P], rho[c], p.dz[k + 1], p.dz[k]) : q == 1 ? rho[c] : FastDiv<T>::prep1(rho[c]);
+        });
+    }
     for (int t = 0; t < 3; t++) {
-        field(a.trc[t], SK_NT, SK_S, 0, nx + 1, nz,
-              [&](int k, int i) { return a.tr.q_old[t][MOIST_IDX(k, i)] / rho[MOIST_IDX(k, i)]; });
-        field(a.trc[t], SK_NT, SK_Q0, 0, nx - 1, nz, [&](int k, int i) { return a.tr.q0[t][MOIST_IDX(k, i)]; });
-        field(a.trc[t], SK_NT, SK_DPH, 0, nx - 1, nz, [&](int k, int i) { return a.tr.dphys[t][MOIST_IDX(k, i)]; });
+        const Field f[SK_BATCH] = {{a.trc[t], SK_NT, SK_S, 0, nx + 1, nz, 2, 0},
+                                   {a.trc[t], SK_NT, SK_Q0, 0, nx - 1, nz, 0, 0},
+                                   {a.trc[t], SK_NT, SK_DPH, 0, nx - 1, nz, 0, 0}};
+        fields(f, [&](int q, int k, int i) {
+            const size_t c = MOIST_IDX(k, i);
+            return q == 0 ? a.tr.q_old[t][c] / rho[c] : q == 1 ? a.tr.q0[t][c] : a.tr.dphys[t][c];
+        });
     }
 }
 template <class T>
@@ -96,127 +135,189 @@ __device__ __forceinline__ void cp_async16(void* s, const void* g) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(sa), "l"(g) : "memory");
 }
 
-// shared memory of one sweep: the ring of records, then the updated values of the two top rows of
-// every warp ([2][warps][STREAM_RING])
+// shared memory of one sweep: per warp its ring of records, the updated values of its two top rows
+// ([2][STREAM_TOP]) and two counts: columns done by its top row, steps begun
+constexpr int SK_REC = (SK_ND + SK_NT) * SK_ROWS;  // elements of a record
 template <class T>
 __host__ __device__ inline size_t stream_smem_bytes(int nz) {
-    return ((size_t)STREAM_RING * (SK_ND + SK_NT) * skew_pitch(nz) + 2 * ((nz + WROWS - 1) / WROWS) * STREAM_RING) * sizeof(T);
+    return (size_t)stream_groups(nz) * ((STREAM_RING * SK_REC + 2 * STREAM_TOP) * sizeof(T) + 2 * sizeof(int));
 }
-inline int stream_threads(int nz) { return (nz + WROWS - 1) / WROWS * 32; }
+inline int stream_threads(int nz) { return stream_groups(nz) * 32; }
+constexpr long long STREAM_SPIN = 4000000000ll;  // bound of a wait for the neighbouring warp, in SM clock cycles (about 2 s)
 
 // one tracer t of one domain; blockDim.x = stream_threads(nz) or more. Returns (to every thread)
 // whether the fast division refused an operand or a result is not finite.
 template <class D, class T>
-__device__ __forceinline__ bool stream_sweep(const DevParams<T>& p, const StreamArgs<T>& a, int t, T* smem) {
-    const int nx = p.nx, nz = p.nz, P = p.P, np = skew_pitch(nz);
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, nwarp = (nz + WROWS - 1) / WROWS;
-    const int r = lane & (WROWS - 1), k = WROWS * wid + r;
-    const bool zh = lane >= WROWS, row_ok = k < nz;
-    const int recd = SK_ND * np, rect = SK_NT * np, rec = recd + rect;
-    T* top1 = smem + (size_t)STREAM_RING * rec;  // [warp][STREAM_RING]: row 16w+15
-    T* top2 = top1 + nwarp * STREAM_RING;        // row 16w+14
-    const T* gd = a.dom;
-    const T* gt = a.trc[t];
-    constexpr int EPC = 16 / sizeof(T);  // elements per 16-byte copy
-    // record s (>= -1) into its slot of the ring; every thread commits one group per call
-    auto issue = [&](int s) {
-        T* dst = smem + (size_t)((s + 1) & (STREAM_RING - 1)) * rec;
-        const T* sd = gd + (size_t)(s + 1) * recd;
-        const T* st = gt + (size_t)(s + 1) * rect;
-        for (int j = threadIdx.x; j < recd / EPC; j += blockDim.x) cp_async16(dst + j * EPC, sd + j * EPC);
-        for (int j = threadIdx.x; j < rect / EPC; j += blockDim.x) cp_async16(dst + recd + j * EPC, st + j * EPC);
-        cp_async_commit();
-    };
-    const HalfRow<T> w = half_row(p, k, zh, a.tr.dt);
-    const T* qo = a.tr.q_old[t];
-    const T lin_km1 = (k - 1 >= 0 && k - 1 < nz) ? qo[MOIST_IDX(k - 1, nx - 2)] : T(0);
-    const T lin_k = row_ok ? qo[MOIST_IDX(k, nx - 2)] : T(0);
-    const T lin_kp1 = (k + 1 < nz) ? qo[MOIST_IDX(k + 1, nx - 2)] : T(0);
-    // this half's clamp rows (z half only)
-    const bool clamp_p = zh && row_ok && (k == 0 || k == nz - 2) && k < nz - 1;
-    const bool clamp_m = zh && row_ok && (k == 1 || k == nz - 1) && k >= 1;
-    // the updated values of the two columns to the left; the seam reads the stage-start values
-    T prev1 = row_ok ? qo[MOIST_IDX(k, nx - 1)] / a.tr.rho[MOIST_IDX(k, nx - 1)] : T(0);
-    T prev2 = row_ok ? qo[MOIST_IDX(k, nx - 2)] / a.tr.rho[MOIST_IDX(k, nx - 2)] : T(0);
-    T sn_last = T(0), m1_used = T(0);
-    T* qn = a.tr.q_new[t] + (size_t)(row_ok ? k : 0) * P;
-    const int z = zh ? 1 : 0, ki = min(k, nz - 1);  // the last warp's rows beyond the domain read row nz-1's inputs
-    const int o_v = (zh ? SK_VZ : SK_VX) * np + ki + 1, o_r = (zh ? SK_RZ : SK_RX) * np + ki + 1;
-    const int o_rho = SK_RHO * np + ki + 1, o_rr = SK_RRHO * np + ki + 1;
-    const int o_s = recd + SK_S * np + ki + 1, o_q = recd + SK_Q0 * np + ki + 1, o_d = recd + SK_DPH * np + ki + 1;
-    const bool in = wid < nwarp;  // warps beyond the rows only copy and meet the barrier
-    bool bad_any = false;
-    struct Ops {
-        T sc, p1, p2, vp, vm, rp, rm, q0, dph, rho, rrho;
-    };
-    auto load = [&](int s) {  // the operands of step s (records s - 1 .. s + 2)
-        auto R = [&](int j) { return smem + (size_t)((j + 1) & (STREAM_RING - 1)) * rec; };
-        const T *R0 = R(s), *Rm = R(s - 1);
-        Ops o;
-        o.sc = R0[o_s];
-        o.p1 = R(s + 1)[o_s + z];
-        o.p2 = R(s + 2)[o_s + 2 * z];
-        o.vp = R0[o_v];
-        o.vm = Rm[o_v - z];
-        o.rp = R0[o_r];
-        o.rm = Rm[o_r - z];
-        o.q0 = R0[o_q];
-        o.dph = R0[o_d];
-        o.rho = R0[o_rho];
-        o.rrho = R0[o_rr];
-        return o;
-    };
-
-    const int nsteps = nx + nz - 1;
-    for (int s = -1; s <= STREAM_RING - 3; s++) issue(s);
-    cp_async_wait<STREAM_RING - 5>();  // records up to 2
-    __syncthreads();
-    Ops nxt = load(0);
-    for (int step = 0; step < nsteps; step++) {
-        // records up to step + 3 have landed (the next step's operands, read one step ahead); the slot of record
-        // step - 2, which nobody reads any more, takes record step + 6 (records beyond the last are allocated)
-        cp_async_wait<STREAM_RING - 6>();
-        __syncthreads();
-        issue(step + STREAM_RING - 2);
-        if (!in) continue;
-        const int c = step - k;
-        const bool active = row_ok && c >= 0 && c < nx;
-        const Ops o = nxt;
-        nxt = load(step + 1);
-        // neighbours: row k-1 stands one column ahead
-        const T up_sn = __shfl_up_sync(0xffffffffu, sn_last, 1);
-        const T up_m1 = __shfl_up_sync(0xffffffffu, m1_used, 1);
-        const int slot = c & (STREAM_RING - 1);
-        const T t1 = wid > 0 ? top1[(wid - 1) * STREAM_RING + slot] : T(0);
-        const T t2 = wid > 0 ? top2[(wid - 1) * STREAM_RING + slot] : T(0);
-        const T m1 = zh ? (r == 0 ? t1 : up_sn) : prev1;
-        const T m2 = zh ? (r == 0 ? t2 : (r == 1 ? t1 : up_m1)) : prev2;
-        T q, sn;
-        bool bad = false;
-        if (__any_sync(0xffffffffu, active && (clamp_p || clamp_m || !(fabs(o.vp) > w.EPS) || !(fabs(o.vm) > w.EPS)))) {
-            // the clamp quotients of limited_flux_z, on the four rows that can use them
-            T cl_p = T(0), cl_m = T(0);
-            if (clamp_p) cl_p = o.vp > w.EPS ? lin_k / (o.vp * p.dt) : lin_kp1 / (-o.vp * p.dt);
-            if (clamp_m) cl_m = o.vm > w.EPS ? lin_km1 / (o.vm * p.dt) : lin_k / (-o.vm * p.dt);
-            two_lane_cell<D, true>(w, m2, m1, o.sc, o.p1, o.p2, o.vp, o.vm, o.rp, o.rm, cl_p, cl_m, o.q0, o.dph, o.rho,
-                                   o.rrho, q, sn, bad);
-        } else {
-            two_lane_cell<D, false>(w, m2, m1, o.sc, o.p1, o.p2, o.vp, o.vm, o.rp, o.rm, T(0), T(0), o.q0, o.dph, o.rho,
-                                    o.rrho, q, sn, bad);
-        }
-        bad_any |= bad && active;
-        if (active && !zh) {
-            qn[c] = q;
-            if (r == WROWS - 1) top1[wid * STREAM_RING + slot] = sn;
-            if (r == WROWS - 2) top2[wid * STREAM_RING + slot] = sn;
-        }
-        prev2 = active ? prev1 : prev2;
-        prev1 = active ? sn : prev1;
-        // lane r+1 reads these next step only for the column it shares with this step
-        sn_last = sn;
-        m1_used = m1;
+__device__ __forceinline__ bool stream_sweep(const DevParams<T>& p, const StreamArgs<T>& a, int t, T* smem, int* timeout) {
+    const int nx = p.nx, nz = p.nz, P = p.P;
+    const int lane = threadIdx.x & 31, g = threadIdx.x >> 5, ng = stream_groups(nz);
+    T* const ring = smem + (size_t)g * (STREAM_RING * SK_REC);
+    T* const tops = smem + (size_t)ng * (STREAM_RING * SK_REC);
+    volatile int* const done = reinterpret_cast<volatile int*>(tops + (size_t)ng * 2 * STREAM_TOP);  // [ng], then begun [ng]
+    volatile int* const begun = done + ng;
+    if (g < ng && lane == 0) {
+        done[g] = 0;
+        begun[g] = 0;
     }
-    cp_async_wait<0>();
+    __syncthreads();
+    bool bad_any = false;
+    if (g < ng) {
+        const int r = lane & (WROWS - 1), k = WROWS * g + r;
+        const bool zh = lane >= WROWS, row_ok = k < nz;
+        T* const top_out = tops + (size_t)g * 2 * STREAM_TOP;                       // row 15, then row 14
+        const T* const top_in = tops + (size_t)(g > 0 ? g - 1 : 0) * 2 * STREAM_TOP;
+        // 16-byte copies: this lane's chunks lane and lane + 32 of a record (domain part, then tracer part)
+        constexpr int EPC = 16 / sizeof(T), CD = SK_ND * SK_ROWS / EPC, CR = SK_REC / EPC;
+        static_assert(CR <= 96, "three chunks a lane at most");
+        const T* gd = a.dom + (size_t)g * skew_records(nx) * (SK_ND * SK_ROWS);
+        const T* gt = a.trc[t] + (size_t)g * skew_records(nx) * (SK_NT * SK_ROWS);
+        const T* src[3];
+        int inc[3];
+#pragma unroll
+        for (int q = 0; q < 3; q++) {
+            const int ch = lane + 32 * q;
+            src[q] = ch < CD ? gd + ch * EPC : gt + (ch - CD) * EPC;
+            inc[q] = ch < CD ? SK_ND * SK_ROWS : SK_NT * SK_ROWS;
+        }
+        auto issue = [&](int slot) {  // the next record into a slot; one group
+            T* dst = ring + slot * SK_REC + lane * EPC;
+#pragma unroll
+            for (int q = 0; q < (CR + 31) / 32; q++)
+                if (lane + 32 * q < CR) {
+                    cp_async16(dst + 32 * q * EPC, src[q]);
+                    src[q] += inc[q];
+                }
+            cp_async_commit();
+        };
+        const HalfRow<T> w = half_row(p, k, zh, a.tr.dt);
+        const T* qo = a.tr.q_old[t];
+        const T lin_km1 = (k - 1 >= 0 && k - 1 < nz) ? qo[MOIST_IDX(k - 1, nx - 2)] : T(0);
+        const T lin_k = row_ok ? qo[MOIST_IDX(k, nx - 2)] : T(0);
+        const T lin_kp1 = (k + 1 < nz) ? qo[MOIST_IDX(k + 1, nx - 2)] : T(0);
+        // this half's clamp rows (z half only)
+        const bool clamp_p = zh && row_ok && (k == 0 || k == nz - 2) && k < nz - 1;
+        const bool clamp_m = zh && row_ok && (k == 1 || k == nz - 1) && k >= 1;
+        const int clamp_g = (nz - 2) / WROWS;  // rows nz-2 and nz-1 lie in this group and above
+        // the updated values of the two columns to the left; the seam reads the stage-start values
+        T prev1 = row_ok ? qo[MOIST_IDX(k, nx - 1)] / a.tr.rho[MOIST_IDX(k, nx - 1)] : T(0);
+        T prev2 = row_ok ? qo[MOIST_IDX(k, nx - 2)] / a.tr.rho[MOIST_IDX(k, nx - 2)] : T(0);
+        T sn_last = T(0), m1_used = T(0);
+        T* qn = a.tr.q_new[t] + (size_t)(row_ok ? k : 0) * P;
+        const int z = zh ? 1 : 0;
+        const int o_v = (zh ? SK_VZ : SK_VX) * SK_ROWS + r + 1, o_r = (zh ? SK_RZ : SK_RX) * SK_ROWS + r + 1;
+        const int o_s = (SK_ND + SK_S) * SK_ROWS + r + 1;
+        struct Ops {
+            T sc, p1, p2, vp, vm, rp, rm, q0, dph, rho, rrho, cl_p, cl_m;
+            bool cen;
+        };
+        auto load = [&](int j) {  // the operands of step j (records j .. j + 3)
+            auto R = [&](int i) { return ring + (i & (STREAM_RING - 1)) * SK_REC; };
+            const T *Rm = R(j), *R0 = R(j + 1);
+            Ops o;
+            o.sc = R0[o_s];
+            o.p1 = R(j + 2)[o_s + z];
+            o.p2 = R(j + 3)[o_s + 2 * z];
+            o.vp = R0[o_v];
+            o.vm = Rm[o_v - z];
+            o.rp = R0[o_r];
+            o.rm = Rm[o_r - z];
+            o.q0 = R0[(SK_ND + SK_Q0) * SK_ROWS + r + 1];
+            o.dph = R0[(SK_ND + SK_DPH) * SK_ROWS + r + 1];
+            o.rho = R0[SK_RHO * SK_ROWS + r + 1];
+            o.rrho = R0[SK_RRHO * SK_ROWS + r + 1];
+            // the clamp quotients of limited_flux_z, on the four rows that can use them, and whether a cell of
+            // the step needs the centred face values: a step ahead, off the chain
+            const bool act = row_ok && j >= r && j - r < nx;
+            o.cl_p = o.cl_m = T(0);
+            o.cen = __any_sync(0xffffffffu, act && (clamp_p || clamp_m || !(fabs(o.vp) > w.EPS) || !(fabs(o.vm) > w.EPS)));
+            if (o.cen && (g == 0 || g >= clamp_g)) {
+                // selected only where |vel| > EPS; IEEE division here, whose quotients of zero and tiny water take
+                // its slow path, made the two warps with clamp rows twice as slow as the others
+                bool bad_p = false, bad_m = false;
+                const T up_p = o.vp > w.EPS ? lin_k : lin_kp1, up_m = o.vm > w.EPS ? lin_km1 : lin_k;
+                o.cl_p = D::quot_var(up_p, fabs(o.vp) * p.dt, bad_p);
+                o.cl_m = D::quot_var(up_m, fabs(o.vm) * p.dt, bad_m);
+                bad_any |= act && ((clamp_p && bad_p && fabs(o.vp) > w.EPS) || (clamp_m && bad_m && fabs(o.vm) > w.EPS));
+            }
+            return o;
+        };
+        // lane 0 waits until *count reaches least (bounded); false: it did not
+        auto wait = [&](const volatile int* count, int least) {
+            int ok = 1;
+            if (lane == 0 && *count < least) {
+                const long long t0 = clock64();
+                while (*count < least)
+                    if (clock64() - t0 > STREAM_SPIN) {
+                        ok = 0;
+                        atomicExch(timeout, 1);
+                        break;
+                    }
+            }
+            ok = __shfl_sync(0xffffffffu, ok, 0);
+            __threadfence_block();  // the values counted are read after the count
+            return ok != 0;
+        };
+        for (int i = 0; i < STREAM_RING; i++) issue(i);
+        cp_async_wait<4>();  // records up to 3
+        __syncwarp();
+        Ops nxt = load(0);
+        const int nsteps = nx + WROWS - 1;
+        for (int j = 0; j < nsteps; j++) {
+            if ((j & (STREAM_HAND - 1)) == 0) {
+                // columns below j - 14 are done by the top row; the warp above may need them, the warp below must
+                // have done the columns of this round, the warp above used those that it overwrites
+                __syncwarp();
+                if (lane == 0) {
+                    __threadfence_block();
+                    done[g] = min(max(j - (WROWS - 1), 0), nx);
+                    begun[g] = j;
+                }
+                if (g > 0 && !wait(done + g - 1, min(j + STREAM_HAND, nx))) break;
+                if (g + 1 < ng && !wait(begun + g + 1, min(j + STREAM_HAND - (WROWS - 2) - STREAM_TOP + 2, nx))) break;
+            }
+            const Ops o = nxt;
+            __syncwarp();  // every lane has read record j
+            issue(j & (STREAM_RING - 1));
+            cp_async_wait<4>();  // records up to j + 4
+            __syncwarp();
+            nxt = load(j + 1);
+            const int c = j - r;
+            const bool active = row_ok && c >= 0 && c < nx;
+            // neighbours: row k-1 stands one column ahead
+            const T up_sn = __shfl_up_sync(0xffffffffu, sn_last, 1);
+            const T up_m1 = __shfl_up_sync(0xffffffffu, m1_used, 1);
+            const int slot = c & (STREAM_TOP - 1);
+            const T t1 = g > 0 ? top_in[slot] : T(0);
+            const T t2 = g > 0 ? top_in[STREAM_TOP + slot] : T(0);
+            const T m1 = zh ? (r == 0 ? t1 : up_sn) : prev1;
+            const T m2 = zh ? (r == 0 ? t2 : (r == 1 ? t1 : up_m1)) : prev2;
+            T q, sn;
+            bool bad = false;
+            if (o.cen)
+                two_lane_cell<D, true>(w, m2, m1, o.sc, o.p1, o.p2, o.vp, o.vm, o.rp, o.rm, o.cl_p, o.cl_m, o.q0, o.dph,
+                                       o.rho, o.rrho, q, sn, bad);
+            else
+                two_lane_cell<D, false>(w, m2, m1, o.sc, o.p1, o.p2, o.vp, o.vm, o.rp, o.rm, T(0), T(0), o.q0, o.dph,
+                                        o.rho, o.rrho, q, sn, bad);
+            bad_any |= bad && active;
+            if (active && !zh) {
+                qn[c] = q;
+                if (r >= WROWS - 2) top_out[(WROWS - 1 - r) * STREAM_TOP + slot] = sn;
+            }
+            prev2 = active ? prev1 : prev2;
+            prev1 = active ? sn : prev1;
+            // lane r+1 reads these next step only for the column it shares with this step
+            sn_last = sn;
+            m1_used = m1;
+        }
+        __syncwarp();
+        if (lane == 0) {
+            __threadfence_block();
+            done[g] = nx;
+            begun[g] = INT_MAX;
+        }
+        cp_async_wait<0>();
+    }
     return __syncthreads_or(bad_any) != 0;
 }
 
@@ -226,7 +327,8 @@ __device__ __forceinline__ void b_tracer_stream(const DevParams<T>& p, const Str
     extern __shared__ __align__(16) unsigned char smem_raw[];
     if (halted(err)) return;
     T* sm = reinterpret_cast<T*>(smem_raw);
-    if (stream_sweep<FastDiv<T>>(p, a, t, sm)) stream_sweep<IeeeDiv<T>>(p, a, t, sm);
+    int* timeout = const_cast<int*>(err) + 2;
+    if (stream_sweep<FastDiv<T>>(p, a, t, sm, timeout)) stream_sweep<IeeeDiv<T>>(p, a, t, sm, timeout);
 }
 
 // single domain: block t sweeps tracer t

@@ -28,7 +28,7 @@ __device__ __forceinline__ u64 mix64(u64 z) {  // splitmix64 finaliser
     return z ^ (z >> 31);
 }
 
-// c: mismatches of cdiv, quot, ratio(b), ratio(-b); refused by cdiv (not finite); accepted by ratio
+// c: mismatches of cdiv, quot and quot_var, ratio(b), ratio(-b); refused by cdiv (not finite); accepted by ratio
 template <class T>
 __device__ __forceinline__ void check(T a, T b, const Rcp<T>& y, T y1, bool prepared, u64* c) {
     using F = FastDiv<T>;
@@ -40,6 +40,9 @@ __device__ __forceinline__ void check(T a, T b, const Rcp<T>& y, T y1, bool prep
         c[4] += !is_finite(q);
         const T q1 = F::quot(a, b, y1, bad);
         c[1] += !bad && is_finite(q1) && !same(q1, r);
+        bad = false;
+        const T q2 = F::quot_var(a, b, bad);
+        c[1] += !bad && !same(q2, r);
     }
     bad = false;
     const T v = F::ratio(a, b, T(0), bad);
