@@ -539,12 +539,28 @@ __device__ __forceinline__ void tracer_slots(const DevParams<double>& p, const A
     v[23] = k >= 1 ? a.mfz[MOIST_IDX(k - 1, i)] : 0.0;
 }
 
-// partial derivatives of every tracer cell with respect to its 24 reads: J[t][slot][cell]
+// The reverse sweep's inputs by anti-diagonal: record d of tracer t holds, for every row k, what the step
+// d = (nx-1-i) + (nz-1-k) of cell (k, i) reads: lambda of its new value, and the partials of the later cells
+// (k, i+1), (k, i+2), (k+1, i), (k+2, i) with respect to it. Entries without a cell stay zero.
+enum { RV_LN = 0, RV_A1, RV_A2, RV_B1, RV_B2, RV_N };
+__host__ __device__ inline int rev_pitch(int nz) { return (nz + 1) / 2 * 2; }  // 16-byte rows
+__host__ __device__ inline int rev_ring(int nz) { return nz <= 512 ? 8 : 4; }  // records in shared memory
+__host__ __device__ inline size_t rev_rows(int nx, int nz) { return (size_t)nx + nz + 1 + rev_ring(nz); }
+inline size_t rev_smem(int nz) {  // the ring, and mu of the last three steps with two rows of zeros on top
+    return ((size_t)rev_ring(nz) * RV_N * rev_pitch(nz) + 3 * (size_t)(nz + 2)) * sizeof(double);
+}
+
+// partial derivatives of every tracer cell with respect to its 24 reads: J[t][slot][cell], and the
+// reverse sweep's records W
 template <class T>
-__device__ __forceinline__ void b_adj_tr_jac(const DevParams<double>& p, const AdjStage<T>& a, double* J, int bid_x,
-                                             int bid_y, int bid_z) {
+__device__ __forceinline__ void b_adj_tr_jac(const DevParams<double>& p, const AdjStage<T>& a, double* J, double* W,
+                                             int bid_x, int bid_y, int bid_z) {
     ADJ_CELL(k, i);
     const int t = bid_z;
+    const int np = rev_pitch(nz), d0 = (nx - 1 - i) + (nz - 1 - k);
+    double* Wt = W + (size_t)t * rev_rows(nx, nz) * RV_N * np;
+    auto rec = [&](int d, int f, int row) -> double& { return Wt[((size_t)d * RV_N + f) * np + row]; };
+    rec(d0, RV_LN, k) = a.Lqout[t][c];
     double v[TR_SLOTS];
     tracer_slots(p, a, t, k, i, v);
     const size_t fsz = (size_t)nz * P;
@@ -564,7 +580,10 @@ __device__ __forceinline__ void b_adj_tr_jac(const DevParams<double>& p, const A
                 ax_r = ax;
                 dx_r = dfx;
             } else {
-                Jt[(size_t)s * fsz + c] = dt * (-ax + dfx);
+                const double j = dt * (-ax + dfx);
+                Jt[(size_t)s * fsz + c] = j;
+                if (s == 1 && i >= 1) rec(d0 + 1, RV_A1, k) = j;
+                if (s == 2 && i >= 2) rec(d0 + 2, RV_A2, k) = j;
             }
         });
     local_jacobian2<ADJ_DUAL>(
@@ -572,77 +591,71 @@ __device__ __forceinline__ void b_adj_tr_jac(const DevParams<double>& p, const A
         [&](int s, double az, double dfz) {
             const double ax = s == 0 ? ax_c : (s == 11 ? ax_r : 0.0);
             const double dfx = s == 0 ? dx_c : (s == 11 ? dx_r : 0.0);
-            Jt[(size_t)s * fsz + c] = dt * (-(ax + az) + (dfx + dfz));
+            const double j = dt * (-(ax + az) + (dfx + dfz));
+            Jt[(size_t)s * fsz + c] = j;
+            if (s == 5 && k >= 1) rec(d0 + 1, RV_B1, k - 1) = j;
+            if (s == 6 && k >= 2) rec(d0 + 2, RV_B2, k - 2) = j;
         });
 }
 template <class T>
 __global__ void __launch_bounds__(ADJ_THREADS) k_adj_tr_jac(const __grid_constant__ DevParams<double> p,
-                                  const __grid_constant__ AdjStage<T> a, double* J) {
-    b_adj_tr_jac(p, a, J, blockIdx.x, blockIdx.y, blockIdx.z);
+                                  const __grid_constant__ AdjStage<T> a, double* J, double* W) {
+    b_adj_tr_jac(p, a, J, W, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
 // reverse sweep: mu(k,i) = lambda_new(k,i) + sum over the later cells that read the new value
 // of (k, i): (k, i+1) [slot L1], (k, i+2) [L2], (k+1, i) [B1], (k+2, i) [B2]. One block per
 // tracer, thread k owns row k; row k handles column nx-1-(d-(nz-1-k)) at step d, after the rows
-// above it, whose results come through a 3-step ring in shared memory.
-__device__ __forceinline__ void b_adj_tr_rev(int nx, int nz, int P, const double* __restrict__ J, const DP<3>& lam_new,
-                                             const DP<3>& mu, int bid_x, int bid_y, int bid_z) {
-    extern __shared__ double ring[];  // [3][nz]
-    const int t = bid_x;
-    const int k = threadIdx.x;
-    const size_t fsz = (size_t)nz * P;
-    const double* Jt = J + (size_t)t * TR_SLOTS * fsz;
-    const double* JL1 = Jt + 1 * fsz;
-    const double* JL2 = Jt + 2 * fsz;
-    const double* JB1 = Jt + 5 * fsz;
-    const double* JB2 = Jt + 6 * fsz;
-    const double* ln = lam_new.f[t];
+// above it. The step's inputs are one record (b_adj_tr_jac), copied with 16-byte cp.async into a ring of
+// shared memory ahead of its use; with the Jacobian's own layout every lane read other lines (five loads,
+// 300 us for 512 x 96; the chain is a barrier and two dependent FMAs a step).
+__device__ __forceinline__ void b_adj_tr_rev(int nx, int nz, int P, const double* __restrict__ W, const DP<3>& mu,
+                                             int bid_x, int bid_y, int bid_z) {
+    extern __shared__ __align__(16) double rev_sm[];
+    const int t = bid_x, k = threadIdx.x, np = rev_pitch(nz), R = rev_ring(nz), rec = RV_N * np;
+    double* last = rev_sm + (size_t)R * rec;  // [3][nz + 2]
+    for (int j = threadIdx.x; j < 3 * (nz + 2); j += blockDim.x) last[j] = 0.0;
+    const double* src = W + (size_t)t * rev_rows(nx, nz) * rec;
     double* m = mu.f[t];
-    const bool active = k < nz;
-    double mp1 = 0.0, mp2 = 0.0;  // mu(k, i+1), mu(k, i+2)
-    // the next step's inputs, loaded one step ahead (they do not depend on mu)
-    double f_ln = 0.0, f_a1 = 0.0, f_a2 = 0.0, f_b1 = 0.0, f_b2 = 0.0;
-    auto fetch = [&](int i) {
-        const size_t cc = MOIST_IDX(k, i);
-        f_ln = ln[cc];
-        f_a1 = i + 1 < nx ? JL1[cc + 1] : 0.0;
-        f_a2 = i + 2 < nx ? JL2[cc + 2] : 0.0;
-        f_b1 = k + 1 < nz ? JB1[cc + P] : 0.0;
-        f_b2 = k + 2 < nz ? JB2[cc + 2 * P] : 0.0;
-        // a row walks its arrays backwards, one 128-byte line per 16 steps: ask for the line
-        // 16 steps ahead into L1 so that the loads above hit
-        if (i >= 16) {
-            const size_t cf = cc - 16;
-            asm volatile("prefetch.global.L1 [%0];" ::"l"(ln + cf));
-            asm volatile("prefetch.global.L1 [%0];" ::"l"(JL1 + cf + 1));
-            asm volatile("prefetch.global.L1 [%0];" ::"l"(JL2 + cf + 2));
-            if (k + 1 < nz) asm volatile("prefetch.global.L1 [%0];" ::"l"(JB1 + cf + P));
-            if (k + 2 < nz) asm volatile("prefetch.global.L1 [%0];" ::"l"(JB2 + cf + 2 * P));
-        }
+    auto issue = [&](int d) {  // record d into its slot (records beyond the last are allocated)
+        double* dst = rev_sm + (size_t)(d & (R - 1)) * rec;
+        const double* s = src + (size_t)d * rec;
+        for (int j = threadIdx.x; j < rec / 2; j += blockDim.x) cp_async16(dst + 2 * j, s + 2 * j);
+        cp_async_commit();
     };
-    if (active) fetch(nx - 1);
+    double mp1 = 0.0, mp2 = 0.0;  // mu(k, i+1), mu(k, i+2)
+    double *l0 = last, *l1 = last + nz + 2, *l2 = l1 + nz + 2;  // mu of this step, the last, the one before
+    for (int d = 0; d < R - 1; d++) issue(d);
     const int nsteps = nx + nz - 1;
     for (int d = 0; d < nsteps; d++) {
+        // record d has landed, and every thread is done with step d - 1
+        if (R == 8)
+            cp_async_wait<6>();
+        else
+            cp_async_wait<2>();
+        __syncthreads();
+        issue(d + R - 1);  // into the slot of record d - 1
         const int i = nx - 1 - (d - (nz - 1 - k));
-        if (active && i >= 0 && i < nx) {
-            const double l = f_ln, a1 = f_a1, a2 = f_a2, b1 = f_b1, b2 = f_b2;
-            if (i >= 1) fetch(i - 1);
-            double v = l;
-            if (i + 1 < nx) v += mp1 * a1;
-            if (i + 2 < nx) v += mp2 * a2;
-            if (k + 1 < nz) v += ring[((d + 2) % 3) * nz + k + 1] * b1;
-            if (k + 2 < nz) v += ring[((d + 1) % 3) * nz + k + 2] * b2;
+        if (k < nz && i >= 0 && i < nx) {
+            const double* q = rev_sm + (size_t)(d & (R - 1)) * rec + k;
+            double v = fma(mp2, q[RV_A2 * np], q[RV_LN * np]);
+            v = fma(l2[k + 2], q[RV_B2 * np], v);
+            v = fma(mp1, q[RV_A1 * np], v);
+            v = fma(l1[k + 1], q[RV_B1 * np], v);
             m[MOIST_IDX(k, i)] = v;
-            ring[(d % 3) * nz + k] = v;
+            l0[k] = v;
             mp2 = mp1;
             mp1 = v;
         }
-        __syncthreads();
+        double* x = l2;
+        l2 = l1;
+        l1 = l0;
+        l0 = x;
     }
+    cp_async_wait<0>();
 }
-__global__ void k_adj_tr_rev(int nx, int nz, int P, const double* __restrict__ J, const __grid_constant__ DP<3> lam_new,
-                             const __grid_constant__ DP<3> mu) {
-    b_adj_tr_rev(nx, nz, P, J, lam_new, mu, blockIdx.x, blockIdx.y, blockIdx.z);
+__global__ void k_adj_tr_rev(int nx, int nz, int P, const double* __restrict__ W, const __grid_constant__ DP<3> mu) {
+    b_adj_tr_rev(nx, nz, P, W, mu, blockIdx.x, blockIdx.y, blockIdx.z);
 }
 
 // the sweep's lambda contributions to everything read through "old" values, rho, the

@@ -70,7 +70,7 @@ template <class T>
 struct ATrJac {
     DevParams<double> p;
     AdjStage<T> a;
-    double* J;
+    double *J, *W;
 };
 template <class T>
 struct ATrScatter {
@@ -86,8 +86,8 @@ struct ATriFact {
 };
 struct ATrRev {
     int nx, nz, P;
-    const double* J;
-    DP<3> lam, mu;
+    const double* W;
+    DP<3> mu;
 };
 struct ASolve {
     int nx, nz, P;
@@ -148,12 +148,12 @@ struct FAUpdate {
 template <class T>
 struct FATrJac {
     __device__ void operator()(const ATrJac<T>& x, int bx, int by) const {
-        b_adj_tr_jac(x.p, x.a, x.J, bx, by % x.p.nz, by / x.p.nz);
+        b_adj_tr_jac(x.p, x.a, x.J, x.W, bx, by % x.p.nz, by / x.p.nz);
     }
 };
 struct FATrRev {
     __device__ void operator()(const ATrRev& x, int bx, int) const {
-        b_adj_tr_rev(x.nx, x.nz, x.P, x.J, x.lam, x.mu, bx, 0, 0);
+        b_adj_tr_rev(x.nx, x.nz, x.P, x.W, x.mu, bx, 0, 0);
     }
 };
 template <class T>

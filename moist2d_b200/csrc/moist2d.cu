@@ -294,7 +294,7 @@ struct Ctx : CtxBase {
         double *dz, *z, *zf;
         double *Lst[7], *LS0[7], *Lph[5], *seed[7];
         double* acc;  // 16 per-stage accumulators, contiguous (one memset)
-        double *Lqout[3], *mu[3], *J, *LP[2][4];
+        double *Lqout[3], *mu[3], *J, *W, *LP[2][4];
         double *Ta, *Tb, *Tc, *Tcp, *Trd, *Lx, *Ly, *Ltp_rho, *Ltp_rt, *Linc_rho, *Linc_rt, *Lsed;
         double *Lpar, *obj, *prec_w, *stage;
         std::vector<Tape> tapes;             // one per step of a segment, or one
@@ -1430,6 +1430,8 @@ struct Ctx : CtxBase {
                 AL(A.mu[t], fsz);
             }
             AL(A.J, 3 * TR_SLOTS * fsz);
+            AL(A.W, 3 * rev_rows(nx, nz) * RV_N * rev_pitch(nz));
+            CK(cudaFuncSetAttribute(k_adj_tr_rev, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
             for (int q = 0; q < 2; q++)
                 for (int f = 0; f < 4; f++) AL(A.LP[q][f], fsz);
             for (double** f : {&A.Ta, &A.Tb, &A.Tc, &A.Tcp, &A.Trd, &A.Lx, &A.Ly, &A.Ltp_rho, &A.Ltp_rt,
@@ -1579,14 +1581,14 @@ struct Ctx : CtxBase {
             a.Linc_rho = A.Linc_rho;
             a.Linc_rt = A.Linc_rt;
             DP<4> LPc{{A.LP[lp][0], A.LP[lp][1], A.LP[lp][2], A.LP[lp][3]}};
-            const DP<3> lq{{A.Lqout[0], A.Lqout[1], A.Lqout[2]}}, mu{{A.mu[0], A.mu[1], A.mu[2]}};
+            const DP<3> mu{{A.mu[0], A.mu[1], A.mu[2]}};
             if (rec) {
                 rec->put(BK_ZERO, BZero{A.acc, 16 * fsz, bz_blocks(fsz)});
                 rec->put(AK_TRI_COEF, AStage<T>{A.pd, a});
                 rec->put(AK_TRI_FACT, ATriFact{nx, nz, P, A.Ta, A.Tb, A.Tc, A.Tcp, A.Trd});
                 rec->put(AK_UPDATE, AStageLP<T>{A.pd, a, LPc});
-                rec->put(AK_TR_JAC, ATrJac<T>{A.pd, a, A.J});
-                rec->put(AK_TR_REV, ATrRev{nx, nz, P, A.J, lq, mu});
+                rec->put(AK_TR_JAC, ATrJac<T>{A.pd, a, A.J, A.W});
+                rec->put(AK_TR_REV, ATrRev{nx, nz, P, A.W, mu});
                 rec->put(AK_TR_SCATTER, ATrScatter<T>{A.pd, a, A.J, mu});
                 rec->put(AK_MF, AStage<T>{A.pd, a});
             } else {
@@ -1594,8 +1596,8 @@ struct Ctx : CtxBase {
                 k_adj_tri_coef<T><<<gc, b, 0, st>>>(A.pd, a);
                 k_adj_tri_fact<<<gcol, 32, 0, st>>>(nx, nz, P, A.Ta, A.Tb, A.Tc, A.Tcp, A.Trd);
                 k_adj_update<T><<<gc, b, 0, st>>>(A.pd, a, LPc);
-                k_adj_tr_jac<T><<<gc3, b, 0, st>>>(A.pd, a, A.J);
-                k_adj_tr_rev<<<3, (nz + 31) / 32 * 32, 3 * nz * sizeof(double), st>>>(nx, nz, P, A.J, lq, mu);
+                k_adj_tr_jac<T><<<gc3, b, 0, st>>>(A.pd, a, A.J, A.W);
+                k_adj_tr_rev<<<3, (nz + 31) / 32 * 32, rev_smem(nz), st>>>(nx, nz, P, A.W, mu);
                 k_adj_tr_scatter<T><<<gc3, b, 0, st>>>(A.pd, a, A.J, mu);
                 k_adj_mf<T><<<gc, b, 0, st>>>(A.pd, a);
             }
@@ -2158,14 +2160,12 @@ struct BatchImpl : BatchBase {
                 break;
             case AK_TR_REV: {  // one block per member and tracer, the longest sweeps first
                 block = dim3(max_rows);
-                int maxnz = 1;
                 std::vector<int> order;
                 for (int i = 0; i < n; i++)
                     if (in_group(i)) {
                         order.push_back(i);
-                        maxnz = std::max(maxnz, m[i]->nz);
+                        smem = std::max(smem, rev_smem(m[i]->nz));
                     }
-                smem = (size_t)3 * maxnz * sizeof(double);
                 std::stable_sort(order.begin(), order.end(),
                                  [&](int a, int b) { return m[a]->nx + m[a]->nz > m[b]->nx + m[b]->nz; });
                 for (int i : order)
@@ -2613,6 +2613,7 @@ struct BatchImpl : BatchBase {
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
             BCK(cudaFuncSetAttribute(k_batched<SINGLE_ARG(BSub<T, TT>), SINGLE_ARG(FSubAsync<T, TT, 3>), 2>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
+            BCK(cudaFuncSetAttribute(k_batched<ATrRev, FATrRev, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
             BCK(cudaFuncSetAttribute(k_batched<BRd<T>, FRd<T>, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
             BCK(cudaFuncSetAttribute(k_batched_b<BStream<T>, FStream<T>, 2 * STREAM_MAX_ROWS, 1>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
