@@ -159,7 +159,7 @@ struct FATrRev {
 template <class T>
 struct FATrScatter {
     __device__ void operator()(const ATrScatter<T>& x, int bx, int by) const {
-        b_adj_tr_scatter(x.p, x.a, x.J, x.mu, bx, by % x.p.nz, by / x.p.nz);
+        b_adj_tr_scatter(x.p, x.a, x.J, x.mu, bx, by, 0);
     }
 };
 template <class T>

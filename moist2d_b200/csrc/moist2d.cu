@@ -1598,7 +1598,7 @@ struct Ctx : CtxBase {
                 k_adj_update<T><<<gc, b, 0, st>>>(A.pd, a, LPc);
                 k_adj_tr_jac<T><<<gc3, b, 0, st>>>(A.pd, a, A.J, A.W);
                 k_adj_tr_rev<<<3, (nz + 31) / 32 * 32, rev_smem(nz), st>>>(nx, nz, P, A.W, mu);
-                k_adj_tr_scatter<T><<<gc3, b, 0, st>>>(A.pd, a, A.J, mu);
+                k_adj_tr_scatter<T><<<gc, b, 0, st>>>(A.pd, a, A.J, mu);
                 k_adj_mf<T><<<gc, b, 0, st>>>(A.pd, a);
             }
             for (int n = m; n >= 1; n--) {
@@ -2181,8 +2181,7 @@ struct BatchImpl : BatchBase {
                             it.push_back({i, (int)bx, 0});
                     }
                 break;
-            case AK_TR_JAC:
-            case AK_TR_SCATTER:  // by = row + nz * tracer
+            case AK_TR_JAC:  // by = row + nz * tracer
                 block = dim3(ADJ_THREADS);
                 for (int i = 0; i < n; i++)
                     if (in_group(i))
