@@ -2223,7 +2223,7 @@ struct BatchImpl : BatchBase {
                 break;
             case BK_SUB:
                 if (sub_strips)
-                    k_batched<BSub<T, TT>, FSubStrip<T, TT>, 4><<<s.nitems, s.block, s.smem, ls>>>(
+                    k_batched<BSub<T, TT>, FSubStrip<T, TT>, 2><<<s.nitems, s.block, s.smem, ls>>>(
                         s.items, (const BSub<T, TT>*)s.args, FSubStrip<T, TT>{});
                 else if (sub_form == 1)
                     k_batched<BSub<T, TT>, FSubPf<T, TT>, 2><<<s.nitems, s.block, s.smem, ls>>>(
@@ -2604,7 +2604,7 @@ struct BatchImpl : BatchBase {
             BCK(cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, owner->device));
             BCK(cudaFuncSetAttribute(k_batched<SINGLE_ARG(BThomas<T, TT>), SINGLE_ARG(FThomasStrip<T, TT>), 4>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
-            BCK(cudaFuncSetAttribute(k_batched<SINGLE_ARG(BSub<T, TT>), SINGLE_ARG(FSubStrip<T, TT>), 4>,
+            BCK(cudaFuncSetAttribute(k_batched<SINGLE_ARG(BSub<T, TT>), SINGLE_ARG(FSubStrip<T, TT>), 2>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
             BCK(cudaFuncSetAttribute(k_batched<SINGLE_ARG(BSub<T, TT>), SINGLE_ARG(FSubAsync<T, TT, 2>), 3>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, optin));
@@ -2651,7 +2651,24 @@ struct BatchImpl : BatchBase {
             BCK(cudaEventCreateWithFlags(&gjoin[g], cudaEventDisableTiming));
         }
         BCK(cudaEventCreateWithFlags(&gfork, cudaEventDisableTiming));
-        assign_groups(1);
+        // The forms before any autotuning. Up to 128 columns per SM the factorisation and substep run over
+        // column strips: one thread per column leaves the SMs waiting for its chain (6 members, 4600
+        // columns: 6.8 ms a step per column, 4.0 over strips); beyond, one thread per column wins (64 members,
+        // 74000 columns: 24.4 over strips, 16.8 per column), in Float32 best in blocks of 128 with the
+        // registers of three blocks of 256 (form 3; form 4 in blocks of 64: 17.6).
+        DeviceInfo di;
+        BCK(device_info(di));
+        long cols = 0;
+        for (auto* c : m) cols += c->nx;
+        sub_strips = cols <= 128L * di.nsm;
+        if (!sub_strips && sizeof(T) == 4) {
+            sub_form = 3;
+            col_threads = 128;
+        }
+        // While the sweeps of all members and tracers are at most two blocks per SM, a launch lasts as long as
+        // its longest members: four chains of members fill the SMs that the others leave (64 members
+        // 16.8 -> 16.1 ms, 6 members 4.0 -> 3.8); with more, the chains contend for the same SMs.
+        assign_groups(n >= 4 && 3 * n <= 2 * di.nsm ? 4 : 1);
         std::vector<int*> ev(n);
         for (int i = 0; i < n; i++) ev[i] = m[i]->err;
         if (int r = dalloc(&errs, n)) return r;

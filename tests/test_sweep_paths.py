@@ -3,7 +3,7 @@ the tiled tracer sweep in chunks of tile columns (more tiles than fit on the GPU
 mixing ratios that fall through the subnormal range (exact ties of the divisions included) and on a
 grid outside the range of the fast division (every tile and sweep repeated with IEEE division); the
 substep, radiation and column solve at every strip width, on the last partial strip, and the column
-solve's and the substep's repeat with IEEE division."""
+solve's and the substep's repeat with IEEE division; ensembles of more columns than column strips take."""
 import numpy as np
 import pytest
 
@@ -107,3 +107,19 @@ def test_column_solve_strips(T, flags, nz, ncols, dt):
     assert rc == abi.MOIST_OK, msg
     torch.cuda.synchronize()
     assert np.array_equal(dev[0].cpu().numpy(), want)
+
+
+@pytest.mark.parametrize("T,flags", [(np.float32, 0), (np.float32, abi.MOIST_FLAG_TRI_NATIVE), (np.float64, 0)],
+                         ids=["f32-tri64", "f32-tri32", "f64"])
+@pytest.mark.parametrize("shapes", [[(6501, 9), (6397, 12), (6303, 7)],
+                                    [(3905, 7), (3841, 12), (3839, 5), (3840, 9), (3907, 17)]], ids=["3", "5"])
+def test_ensembles_of_many_columns(T, flags, shapes):
+    """More columns than the column strips take by default, in one chain of members and in several."""
+    mem = [small_case(T, nx, nz) for nx, nz in shapes]
+    with model.Ensemble([p for p, _ in mem], flags) as e:
+        for i, (_, s) in enumerate(mem):
+            e.upload(i, s)
+        e.step(3)
+        got = [e.download(i, s.copy()) for i, (_, s) in enumerate(mem)]
+    for (p, s), g in zip(mem, got):
+        compare(g, model.rk3_step(s.copy(), p, 3, flags=flags), p)
