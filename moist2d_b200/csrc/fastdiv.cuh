@@ -50,6 +50,12 @@ __device__ __forceinline__ float sel_u(unsigned c, float x, float y) {  // c != 
 __device__ __forceinline__ bool same_bits(float x, float y) { return __float_as_uint(x) == __float_as_uint(y); }
 __device__ __forceinline__ bool same_bits(double x, double y) { return __double_as_longlong(x) == __double_as_longlong(y); }
 
+// the sign of x flipped where the bit `m` (0 or 0x80000000) is set
+__device__ __forceinline__ float flip(float x, unsigned m) { return __uint_as_float(__float_as_uint(x) ^ m); }
+__device__ __forceinline__ double flip(double x, unsigned m) {
+    return __hiloint2double(__double2hiint(x) ^ (int)m, __double2loint(x));
+}
+
 // Julia's min / max (NaN-propagating, -0 < +0) as single PTX instructions
 __device__ __forceinline__ float jmin_f(float a, float b) {
     float r;
@@ -144,21 +150,21 @@ struct Div64X {  // FP64 reciprocal with explicit rounding of subnormal quotient
 // Let q0 be within one ulp of a/b. Its remainder a - b q0 is then a float (the FMA forms it
 // exactly), and RN(q0 + (a - b q0) RN(1/b)) = RN(a/b) (P. Markstein, IBM J. Res. Dev. 34, 1990;
 // the quotient theorem of Muller et al., Handbook of Floating-Point Arithmetic). The remainder
-// must not underflow: it is formed from the numerator and q0 scaled by UP (both exact), and the
-// last FMA takes it back with RN(1/b) / UP onto the unscaled q0, so a subnormal quotient too is
-// rounded once, onto its own grid. There the argument holds but for exact ties (the rounding
+// must not underflow: it is formed from the numerator and the denominator scaled by UP (both exact,
+// and off the dependent path), and the last FMA takes it back with RN(1/b) / UP onto the unscaled
+// q0, so a subnormal quotient too is rounded once, onto its own grid. There the argument holds but for exact ties (the rounding
 // error of 1/b decides them): a tie is |remainder| = b times half a grid unit. cdiv sends it to the
 // even neighbour (the tails at the edges of clouds fall through the subnormal range within a few
 // cells, where every hundredth or so quotient by 100 or 250 is one); in quot and ratio, whose
 // denominators have long significands, it sets `bad`.
 //   prepared b (cdiv): q0 = RN(a d + RN(a l)) with d + l = 1/b to 2^-40, and one correction;
-//   variable b: RN(1/b) from the hardware approximation, q0 = RN(a RN(1/b)) is within 1.5 ulp,
-//   one correction makes it one of the two values around a/b, a second one RN(a/b).
+//   variable b: with y0 = 1/b to about one ulp, q0 = RN(a y0) is within a few ulps, one correction
+//   with y0 makes it one of the two values around a/b, a second one, with RN(1/b) formed
+//   meanwhile, RN(a/b).
 // d is 1/b rounded down, so that both terms of q0 and the correction of a zero keep the sign of a
 // zero numerator (b > 0). What leaves the admitted ranges ends as a non-finite result or sets
 // `bad`, never as a wrong finite one: a prepared denominator outside [LO, HI] has NaN
-// reciprocals, |a| UP and q0 UP overflow to infinities that the correction turns into an
-// infinity or NaN, a variable denominator above BIG sets `bad`. The sweeps check `bad` and the
+// reciprocals, |a| UP overflows to an infinity that the correction turns into an infinity or NaN, a variable denominator above BIG sets `bad`. The sweeps check `bad` and the
 // finiteness of their results once per tile or sweep and repeat it with IeeeDiv.
 // tests/celldiv_check.cu compares every primitive with IEEE division on the GPU: all 2^32 numerators for
 // the model's denominators, all 2^32 denominators for the reciprocal, and random bit patterns.
@@ -193,21 +199,22 @@ __device__ __forceinline__ double fma_t(double a, double b, double c) { return _
 __device__ __forceinline__ float rcp_rd(float b) { return __frcp_rd(b); }
 __device__ __forceinline__ double rcp_rd(double b) { return __drcp_rd(b); }
 
-// RN(1/b) of a variable denominator: the hardware approximation and Newton steps. Float: one
-// step, checked against IEEE division for every |b| in [2^-125, 2^125]. Double: two steps reach
-// one ulp, the third gives RN(1/b) unless b's significand is all ones (Markstein), which sets bad.
-__device__ __forceinline__ float rcp_rn(float b, bool&) {
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(b));
-    return __fmaf_rn(y, __fmaf_rn(-b, y, 1.0f), y);
+// 1/b of a variable denominator: y0 to about one ulp and RN(1/b). Float: y0 is the hardware
+// approximation and one Newton step gives RN(1/b), checked against IEEE division for every |b| in
+// [2^-125, 2^125]. Double: the cubic step y (1 + e + e e) on the approximation's 20 bits or more
+// reaches one ulp, and a Newton step on it gives RN(1/b) unless b's significand is all ones
+// (Markstein), which sets bad.
+__device__ __forceinline__ float rcp_rn(float b, float& y0, bool&) {
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y0) : "f"(b));
+    return __fmaf_rn(y0, __fmaf_rn(-b, y0, 1.0f), y0);
 }
-__device__ __forceinline__ double rcp_rn(double b, bool& bad) {
+__device__ __forceinline__ double rcp_rn(double b, double& y0, bool& bad) {
     double y;
     asm("rcp.approx.ftz.f64 %0, %1;" : "=d"(y) : "d"(b));
-    y = __fma_rn(y, __fma_rn(-b, y, 1.0), y);
-    y = __fma_rn(y, __fma_rn(-b, y, 1.0), y);
+    const double e = __fma_rn(-b, y, 1.0);
+    y0 = __fma_rn(y, __fma_rn(e, e, e), y);
     bad |= ((unsigned long long)__double_as_longlong(b) << 12) == 0xfffffffffffff000ull;
-    return __fma_rn(y, __fma_rn(-b, y, 1.0), y);
+    return __fma_rn(y0, __fma_rn(-b, y0, 1.0), y0);
 }
 
 template <class T>
@@ -225,50 +232,48 @@ struct FastDiv : DivRange<T> {
     __device__ __forceinline__ static T prep1(T b) { return b >= DR::LO && b <= DR::HI ? T(1) / b : T(0) / T(0); }
     __device__ __forceinline__ static T cdiv(T a, T b, const Rcp<T>& y) {
         const T q0 = fma_t(a, y.d, a * y.l);
-        const T rn = fma_t(b, q0 * DR::UP, -(a * DR::UP));  // negated: +0 for a zero of either sign
+        const T rn = fma_t(b * DR::UP, q0, -(a * DR::UP));  // negated: +0 for a zero of either sign
         // on a tie the correction with a slightly larger reciprocal reaches the other neighbour
         const T other = fma_t(-rn, y.n * T(1.0000305), q0);
         return fabs(rn) == y.tie ? (odd(q0) ? other : q0) : fma_t(-rn, y.n, q0);
     }
-    __device__ __forceinline__ static T twice(T a, T b, T y, T tie, bool& bad) {
-        const T as = -(a * DR::UP), n = y * DR::DOWN;
-        T q = a * y;
-        q = fma_t(-fma_t(b, q * DR::UP, as), n, q);
-        const T rn = fma_t(b, q * DR::UP, as);
+    // a / b with y = RN(1/b) and y0 near it
+    __device__ __forceinline__ static T twice(T a, T b, T y0, T y, T tie, bool& bad) {
+        const T as = -(a * DR::UP), bs = b * DR::UP;
+        T q = a * y0;
+        q = fma_t(-fma_t(bs, q, as), y0 * DR::DOWN, q);
+        const T rn = fma_t(bs, q, as);
         bad |= fabs(rn) == tie;
-        return fma_t(-rn, n, q);
+        return fma_t(-rn, y * DR::DOWN, q);
     }
     // a / b with y = prep1(b)
-    __device__ __forceinline__ static T quot(T a, T b, T y, bool& bad) { return twice(a, b, y, b * DR::TIE, bad); }
+    __device__ __forceinline__ static T quot(T a, T b, T y, bool& bad) { return twice(a, b, y, y, b * DR::TIE, bad); }
     // a / b for a variable b > 0; a result that is not finite sets bad
     __device__ __forceinline__ static T quot_var(T a, T b, bool& bad) {
-        const T q = twice(a, b, rcp_rn(b, bad), b * DR::TIE, bad);
+        T y0;
+        const T y = rcp_rn(b, y0, bad);
+        const T q = twice(a, b, y0, y, b * DR::TIE, bad);
         bad |= b > DR::BIG || !(fabs(q) <= DR::MAX);
         return q;
     }
-    // the limiter ratio: |b| < EPS ? 1 : a / b (the sign of a zero is not kept for b < 0: the limiter
-    // takes both zeros to +0)
-    __device__ __forceinline__ static T ratio(T a, T b, T EPS, bool& bad) {
+    // the limiter ratio a / b, not used where `one` (the sign of a zero is not kept for b < 0: the
+    // limiter takes both zeros to +0)
+    __device__ __forceinline__ static T ratio(T a, T b, bool one, bool& bad) {
         const T ab = fabs(b);
-        const bool one = ab < EPS;
         bool refuse = ab > DR::BIG;
-        const T y = rcp_rn(b, refuse);
-        const T q = twice(a, b, y, ab * DR::TIE, refuse);
+        T y0;
+        const T y = rcp_rn(b, y0, refuse);
+        const T q = twice(a, b, y0, y, ab * DR::TIE, refuse);
         bad |= !one && refuse;
-        return one ? T(1) : q;
+        return q;
     }
-    // (1 + 2 r) / 3: the numerator is 0 or at least 2^-24 (2^-53) in magnitude. Float: 1/3 as two
-    // floats and one FMA, checked for every numerator of 2^-30 to 2^120.
-    __device__ __forceinline__ static T div3(T a) {
-        if constexpr (sizeof(T) == 4) {
-            constexpr float yh = 1.0f / 3.0f, yl = (float)(1.0 / 3.0 - (double)yh);
-            return __fmaf_rn(a, yh, a * yl);
-        } else {
-            constexpr double y = 1.0 / 3.0;
-            double q = a * y;
-            q = __fma_rn(__fma_rn(-3.0, q, a), y, q);
-            return __fma_rn(__fma_rn(-3.0, q, a), y, q);
-        }
+    // (1 + 2 r) / 6: the numerator is 0 or at least 2^-24 (2^-53) in magnitude. 1/6 as the sum of two
+    // values of the type, good to twice its precision: a quotient by 6 that is no tie lies a twelfth
+    // of an ulp or more from every rounding boundary, and there are no ties but subnormal ones.
+    __device__ __forceinline__ static T div6(T a) {
+        constexpr T yh = T(1) / T(6);  // RN(1/6), and the rest exactly (1 - 6 yh) / 6
+        constexpr T yl = sizeof(T) == 4 ? T(1.0 / 6.0 - (double)yh) : yh * T(0x1p-54);
+        return fma_t(a, yh, a * yl);
     }
 };
 
@@ -278,8 +283,8 @@ struct IeeeDiv {
     __device__ __forceinline__ static T cdiv(T a, T b, const Rcp<T>&) { return a / b; }
     __device__ __forceinline__ static T quot(T a, T b, T, bool&) { return a / b; }
     __device__ __forceinline__ static T quot_var(T a, T b, bool&) { return a / b; }
-    __device__ __forceinline__ static T ratio(T a, T b, T EPS, bool&) { return fabs(b) < EPS ? T(1) : a / b; }
-    __device__ __forceinline__ static T div3(T a) { return a / T(3); }
+    __device__ __forceinline__ static T ratio(T a, T b, bool, bool&) { return a / b; }
+    __device__ __forceinline__ static T div6(T a) { return a / T(6); }
 };
 
 // ---- the correctly rounded double quotient a/b without a division on the dependent path

@@ -128,9 +128,10 @@ __global__ void __launch_bounds__(kThreads) k_implicit_columns_noalloc(int nz, i
         bool bad = false;
         eliminate([&](TT c, TT num, TT piv, TT& q_c, TT& q_d) {
             bad |= !(piv >= F::LO && piv <= F::HI);
-            const TT y = moist::rcp_rn(piv, bad);
-            q_c = F::twice(c, piv, y, piv * F::TIE, bad);
-            q_d = F::twice(num, piv, y, piv * F::TIE, bad);
+            TT y0;
+            const TT y = moist::rcp_rn(piv, y0, bad);
+            q_c = F::twice(c, piv, y0, y, piv * F::TIE, bad);
+            q_d = F::twice(num, piv, y0, y, piv * F::TIE, bad);
             bad |= !(fabs(q_c) <= F::MAX) || !(fabs(q_d) <= F::MAX);
         });
         if (bad)

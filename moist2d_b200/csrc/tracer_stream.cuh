@@ -197,6 +197,7 @@ __device__ __forceinline__ bool stream_sweep(const DevParams<T>& p, const Stream
         // this half's clamp rows (z half only)
         const bool clamp_p = zh && row_ok && (k == 0 || k == nz - 2) && k < nz - 1;
         const bool clamp_m = zh && row_ok && (k == 1 || k == nz - 1) && k >= 1;
+        const bool edge = clamp_p || clamp_m || (zh && row_ok && (k == 0 || k == nz - 1));
         const int clamp_g = (nz - 2) / WROWS;  // rows nz-2 and nz-1 lie in this group and above
         // the updated values of the two columns to the left; the seam reads the stage-start values
         T prev1 = row_ok ? qo[MOIST_IDX(k, nx - 1)] / a.tr.rho[MOIST_IDX(k, nx - 1)] : T(0);
@@ -229,7 +230,7 @@ __device__ __forceinline__ bool stream_sweep(const DevParams<T>& p, const Stream
             // the step needs the centred face values: a step ahead, off the chain
             const bool act = row_ok && j >= r && j - r < nx;
             o.cl_p = o.cl_m = T(0);
-            o.cen = __any_sync(0xffffffffu, act && (clamp_p || clamp_m || !(fabs(o.vp) > w.EPS) || !(fabs(o.vm) > w.EPS)));
+            o.cen = __any_sync(0xffffffffu, act && (edge || !(fabs(o.vp) > w.EPS) || !(fabs(o.vm) > w.EPS)));
             if (o.cen && (g == 0 || g >= clamp_g)) {
                 // selected only where |vel| > EPS; IEEE division here, whose quotients of zero and tiny water take
                 // its slow path, made the two warps with clamp rows twice as slow as the others

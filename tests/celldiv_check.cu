@@ -4,10 +4,10 @@
 //
 //   cdiv b...        every float numerator by each b > 0: "<b> <cdiv> <quot> <ratio> <ratio by -b> <bad>"
 //   rcp              rcp_rn of every float |b| in [2^-125, 2^125] against 1/b: "rcp <mismatches>"
-//   div3             every float numerator of |a| in [2^-30, 2^120], and +0: "div3 <mismatches>"
+//   div6             every float numerator of |a| in [2^-30, 2^120], and +0: "div6 <mismatches>"
 //   random n seed    n random float (a, b) bit patterns, half of them with exponents near the type's
 //                    lower end: "random <cdiv> <quot> <ratio> <accepted>"
-//   random64 n seed  the same in double, with div3: "random64 <cdiv> <quot> <ratio> <div3> <accepted>"
+//   random64 n seed  the same in double, with div6: "random64 <cdiv> <quot> <ratio> <div6> <accepted>"
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
@@ -45,11 +45,11 @@ __device__ __forceinline__ void check(T a, T b, const Rcp<T>& y, T y1, bool prep
         c[1] += !bad && !same(q2, r);
     }
     bad = false;
-    const T v = F::ratio(a, b, T(0), bad);
+    const T v = F::ratio(a, b, false, bad);
     c[2] += !bad && is_finite(v) && v != r;
     c[5] += !bad && is_finite(v);
     bad = false;
-    const T w = F::ratio(a, -b, T(0), bad);
+    const T w = F::ratio(a, -b, false, bad);
     c[3] += !bad && is_finite(w) && w != -r;
 }
 
@@ -67,17 +67,18 @@ __global__ void k_rcp(u64* out) {
     u64 n = 0;
     for (u64 u = blockIdx.x * (u64)blockDim.x + threadIdx.x; u < (1ull << 32); u += st) {
         const float b = __uint_as_float((unsigned)u);
+        float y0;
         bool bad = false;
-        if (fabsf(b) >= 0x1p-125f && fabsf(b) <= 0x1p125f) n += !same(rcp_rn(b, bad), 1.0f / b);
+        if (fabsf(b) >= 0x1p-125f && fabsf(b) <= 0x1p125f) n += !same(rcp_rn(b, y0, bad), 1.0f / b);
     }
     atomicAdd(out, n);
 }
-__global__ void k_div3(u64* out) {
+__global__ void k_div6(u64* out) {
     const u64 st = (u64)gridDim.x * blockDim.x;
     u64 n = 0;
     for (u64 u = blockIdx.x * (u64)blockDim.x + threadIdx.x; u < (1ull << 32); u += st) {
         const float a = __uint_as_float((unsigned)u);
-        if (u == 0 || (fabsf(a) >= 0x1p-30f && fabsf(a) <= 0x1p120f)) n += !same(FastDiv<float>::div3(a), a / 3.0f);
+        if (u == 0 || (fabsf(a) >= 0x1p-30f && fabsf(a) <= 0x1p120f)) n += !same(FastDiv<float>::div6(a), a / 6.0f);
     }
     atomicAdd(out, n);
 }
@@ -96,7 +97,7 @@ __global__ void k_random(u64 n, u64 seed, u64* out) {
 }
 __global__ void k_random64(u64 n, u64 seed, u64* out) {
     const u64 st = (u64)gridDim.x * blockDim.x;
-    u64 c[6] = {0, 0, 0, 0, 0, 0}, d3 = 0;
+    u64 c[6] = {0, 0, 0, 0, 0, 0}, d6 = 0;
     for (u64 j = blockIdx.x * (u64)blockDim.x + threadIdx.x; j < n; j += st) {
         u64 ua = mix64(seed * 0x9e3779b97f4a7c15ull + 2 * j), ub = mix64(seed * 0x9e3779b97f4a7c15ull + 2 * j + 1);
         if (j & 1) ub = (ub & 0x800fffffffffffffull) | ((((ub >> 52) & 0x1f) + 1007ull) << 52);
@@ -109,10 +110,10 @@ __global__ void k_random64(u64 n, u64 seed, u64* out) {
         const double a = __longlong_as_double((long long)ua), b = fabs(__longlong_as_double((long long)ub));
         check(a, b, FastDiv<double>::prep(b), FastDiv<double>::prep1(b), true, c);
         const double m = __longlong_as_double((long long)((ua & 0x800fffffffffffffull) | ((((ua >> 52) & 0x7f) + 970ull) << 52)));
-        d3 += !same(FastDiv<double>::div3(m), m / 3.0);
+        d6 += !same(FastDiv<double>::div6(m), m / 6.0);
     }
     for (int j = 0; j < 6; j++) atomicAdd(out + j, c[j]);
-    atomicAdd(out + 6, d3);
+    atomicAdd(out + 6, d6);
 }
 
 int main(int argc, char** argv) {
@@ -139,9 +140,9 @@ int main(int argc, char** argv) {
     } else if (!strcmp(mode, "rcp")) {
         run([&] { k_rcp<<<g, b>>>(d); });
         printf("rcp %llu\n", h[0]);
-    } else if (!strcmp(mode, "div3")) {
-        run([&] { k_div3<<<g, b>>>(d); });
-        printf("div3 %llu\n", h[0]);
+    } else if (!strcmp(mode, "div6")) {
+        run([&] { k_div6<<<g, b>>>(d); });
+        printf("div6 %llu\n", h[0]);
     } else if (!strcmp(mode, "random") && argc == 4) {
         run([&] { k_random<<<g, b>>>(strtoull(argv[2], nullptr, 10), strtoull(argv[3], nullptr, 10), d); });
         printf("random %llu %llu %llu %llu\n", h[0], h[1], h[2] + h[3], h[5]);

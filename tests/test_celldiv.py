@@ -36,13 +36,13 @@ def test_every_numerator(checker):
         assert line[:4] == [0, 0, 0, 0] and line[4] == 2 ** 32, b
 
 
-def test_every_denominator_of_the_reciprocal_and_thirds(checker):
+def test_every_denominator_of_the_reciprocal_and_sixths(checker):
     assert run(checker, "rcp") == [[0]]
-    assert run(checker, "div3") == [[0]]
+    assert run(checker, "div6") == [[0]]
 
 
 def test_random_bit_patterns(checker):
     ((cdiv, quot, ratio, accepted),) = run(checker, "random", 1 << 31, 5)
     assert (cdiv, quot, ratio) == (0, 0, 0) and accepted > 1 << 29
-    ((cdiv, quot, ratio, div3, accepted),) = run(checker, "random64", 1 << 30, 6)
-    assert (cdiv, quot, ratio, div3) == (0, 0, 0, 0) and accepted > 1 << 28
+    ((cdiv, quot, ratio, div6, accepted),) = run(checker, "random64", 1 << 30, 6)
+    assert (cdiv, quot, ratio, div6) == (0, 0, 0, 0) and accepted > 1 << 28
