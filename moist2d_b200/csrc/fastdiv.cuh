@@ -1,14 +1,18 @@
-// fastdiv.cuh - branch-free, correctly rounded Float32 division for the tracer sweep.
+// fastdiv.cuh - branch-free, correctly rounded division for the hot loops.
 //
-// CUDA's IEEE division (div.rn.f32) ends every quotient with a range check and a branch to a
-// slow path (very slow for subnormal results), so consecutive divisions cannot overlap and the
-// code between them cannot be scheduled together: a tracer cell update with ~25 divisions costs
-// ~1800 cycles of dependent latency, and the Gauss-Seidel tracer sweep walks long chains of
-// such updates. Here float division is RN32(RN64(a * y)) with y = 1/b in double precision
-// (proof at div64), which returns the IEEE quotient for every input except ties in the
-// subnormal range; those are reported through a guard word (Div64) or rounded explicitly
-// (Div64X). tests/fastdiv_check.cu checks both against IEEE division on the GPU, exhaustively
-// over all numerators for the model's denominators and on random bit patterns of every class.
+// CUDA's IEEE division ends every quotient with a range check and a branch to a slow path (very
+// slow for subnormal results), so consecutive divisions cannot overlap and the code between them
+// cannot be scheduled together: a tracer cell of ~25 such divisions is ~1800 cycles of dependent
+// latency, and the Gauss-Seidel tracer sweep walks long chains of cells. Three policies:
+//   FastDiv<T> (tracer cell, column solve): remainder corrections in the type's own precision; what
+//       it cannot round exactly is reported and the caller repeats with IeeeDiv<T>;
+//   RN32(RN64(a y)) with y = 1/b in double precision (div64; slow tendencies), the IEEE quotient of
+//       floats but for ties in the subnormal range, which a guard word reports (Div64) or explicit
+//       rounding resolves (Div64X);
+//   qdiv_checked / quotient_proven (Thomas recurrences): a corrected double quotient with an exact
+//       acceptance test.
+// tests/fastdiv_check.cu and tests/celldiv_check.cu compare them with IEEE division on the GPU, over
+// all numerators for the model's denominators and on random bit patterns of every class.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -119,7 +123,7 @@ __device__ __forceinline__ double rcp64(float b) {
     return __fma_rn(y, e, y);
 }
 
-// division policies of the fast tracer cell: cdiv(a, b, y, g) with y = 1/b prepared once,
+// division policies by the double reciprocal: cdiv(a, b, y, g) with y = 1/b prepared once,
 // vdiv(a, b, g) for a variable denominator, div3(a) = a / 3; g is the subnormal guard word
 struct Div64 {  // FP64 reciprocal: exact for every input but subnormal ties, which g reports
     using R = double;

@@ -16,8 +16,8 @@
 // values of that warp's two top rows: they pass through a ring of shared memory, with counts of the
 // columns done and used, read and written every STREAM_HAND steps. (With one block barrier a step,
 // and a whole block copying each record, a step took 2500 cycles, of which the cell takes about 500: the
-// slowest warp, and the copies' and the barrier's instructions, for every warp.) Waits on a count
-// are bounded and report through the error words.
+// slowest warp, and the copies' and the barrier's instructions, for every warp: 10.7 ms of a step of 64
+// members, 6.9 this way.) Waits on a count are bounded and report through the error words.
 #pragma once
 
 #include "tracer_tiles.cuh"

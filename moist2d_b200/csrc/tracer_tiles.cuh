@@ -24,7 +24,10 @@
 //
 // What bounds it: the chain of dependent cells. A tile is 47 wavefront steps; with 16 rows and two
 // lanes per cell a step is about half as long as with 32 rows and a lane per cell, a tile needs 47
-// steps instead of 63, and twice as many tiles spread over the SMs.
+// steps instead of 63, and twice as many tiles spread over the SMs. The walk of a whole tile (alone on
+// its SM): 16 us in Float32, 31 us in Float64; the sweeps of a step on 2048 x 128 0.94 -> 0.37 ms in
+// Float32, 11.6 -> 2.7 ms in Float64 (two chunks), on 4096 x 256 (four chunks; one block's wavefront
+// with IEEE division before) 96.7 -> 3.2 ms.
 #pragma once
 
 #include "tracer_cell.cuh"
@@ -68,7 +71,7 @@ __device__ __forceinline__ unsigned long long ld_acquire64(const unsigned long l
 // next barrier on the same counter only after every block has left the one in between. One thread
 // per block arrives with a reduction (nothing returned) and polls without sleeping; the counter
 // costs one round trip to L2 instead of an arrival, a release and a read of a changed flag in turn
-// (4.1 us for a pass without work on 2048 x 128, 512 blocks, before).
+// (a pass without work on 2048 x 128, 512 blocks: 4.1 us before, 3.2 us now).
 struct GridSync {
     unsigned n = 0;                            // barriers so far
     unsigned seen[2] = {0, 0};                 // high words at the end of the last even and odd barrier
