@@ -2665,10 +2665,10 @@ struct BatchImpl : BatchBase {
             sub_form = 3;
             col_threads = 128;
         }
-        // While the sweeps of all members and tracers are at most two blocks per SM, a launch lasts as long as
-        // its longest members: four chains of members fill the SMs that the others leave (64 members
-        // 16.8 -> 16.1 ms, 6 members 4.0 -> 3.8); with more, the chains contend for the same SMs.
-        assign_groups(n >= 4 && 3 * n <= 2 * di.nsm ? 4 : 1);
+        // One chain of launches lasts, launch by launch, as long as its longest members: with four members or
+        // more, four chains fill the SMs that the others leave (6 members 4.0 -> 3.8 ms a step, 64 members
+        // 16.8 -> 16.1, 256 members 45.2 -> 42.2, with two chains 41.9).
+        assign_groups(n >= 4 ? 4 : 1);
         std::vector<int*> ev(n);
         for (int i = 0; i < n; i++) ev[i] = m[i]->err;
         if (int r = dalloc(&errs, n)) return r;
