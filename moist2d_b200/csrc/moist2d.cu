@@ -2882,12 +2882,12 @@ struct BatchImpl : BatchBase {
                 bmb = mb;
             }
         }
-        best = best_mb;
         stream_minb = bmb;
-        // then the number of member groups whose chains run as parallel branches of the graph
-        int bg = 1;
-        float best_g = best;
-        for (int G : {2, 4}) {
+        // then the number of member groups whose chains run as parallel branches of the graph (the
+        // candidates above ran with the groups the batch had): every count is timed, one included
+        int bg = ngroups;
+        float best_g = 1e30f;
+        for (int G : {1, 2, 4}) {
             if (G > (int)m.size()) continue;
             assign_groups(G);
             if (int r = set_col_threads(bct)) return r;  // new work lists and graphs

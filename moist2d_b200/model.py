@@ -322,7 +322,7 @@ class Ensemble:
     def autotune(self, nsteps=2):
         """moist_batch_autotune: time the per-column kernels' block sizes from the current
         States, keep the fastest, restore the States; returns the report."""
-        buf = C.create_string_buffer(1024)
+        buf = C.create_string_buffer(4096)
         self._check(lib().moist_batch_autotune(self.b, int(nsteps), buf, len(buf)), "moist_batch_autotune")
         return buf.value.decode()
 
