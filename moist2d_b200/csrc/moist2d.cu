@@ -898,7 +898,7 @@ struct Ctx : CtxBase {
         tr.mfx = mfx;
         tr.mfz = mfz;
         tr.dt = dt_stage;
-        MARK(MOIST_KGROUP_TRACER, (use_stream || use_tiles) ? 2 : 1);
+        MARK(MOIST_KGROUP_TRACER, use_stream || (use_tiles && tiles_df) ? 2 : 1);
         if (use_stream) {
             StreamArgs<T> sa{tr, skew_dom, {skew_trc[0], skew_trc[1], skew_trc[2]}};
             if (rec) {
