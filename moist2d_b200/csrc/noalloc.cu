@@ -37,6 +37,39 @@ void put_msg(char* err, size_t errlen, const char* msg) {
     }
 }
 
+// One row of the w-p system of a column (moist.jl:974-1030): level k, th, r2, w and dw at that level
+template <class T>
+struct Row {
+    T a, b, c, d;  // the diagonal is b + 1
+};
+template <class T>
+struct Factors {
+    T grav, dt_tp2, fact;
+    __device__ Factors(T grav_, T beta, T dt) : grav(grav_) {
+        const T fact_tp = T(0.5) * (T(1.0) + beta);
+        const T fact_tm = T(0.5) * (T(1.0) - beta);
+        dt_tp2 = (dt * fact_tp) * (dt * fact_tp);
+        fact = fact_tm / fact_tp;
+    }
+};
+template <class T, int CAP>
+__device__ __forceinline__ Row<T> row_of(int k, int ke, const Factors<T>& f, const ColumnGrid<T, CAP>& grid, const T* th,
+                                         const T* r2, const T* w, const T* dw) {
+    const T dz_k = grid.dz[k], dz_kp = grid.dz[k + 1], zd = grid.z[k + 1] - grid.z[k];
+    const T th_cur = moist::f2h(th[0], th[1], dz_k, dz_kp);
+    const T th_prev = k > 0 ? moist::f2h(th[-1], th[0], grid.dz[k - 1], dz_k) : T(0);
+    const T th_next = (k + 1 <= ke - 1) ? moist::f2h(th[1], th[2], dz_kp, grid.dz[k + 2]) : T(0);
+    Row<T> r;
+    r.b = f.dt_tp2 * (r2[0] / dz_k + r2[1] / dz_kp) * th_cur / zd;
+    r.a = (k > 0) ? -f.dt_tp2 * (r2[0] * th_prev / (zd * dz_k) - f.grav / (dz_k + dz_kp)) : T(0);
+    r.c = (k < ke - 1) ? -f.dt_tp2 * (r2[1] * th_next / (zd * dz_kp) + f.grav / (dz_k + dz_kp)) : T(0);
+    r.d = w[0] + dw[0];
+    if (k > 0) r.d -= r.a * f.fact * w[0];
+    r.d -= r.b * f.fact * w[0];
+    if (k < ke - 1) r.d -= r.c * f.fact * w[1];
+    return r;
+}
+
 // shared memory of one level of one column: a, b + 1, c, d (T), c', d' (TT)
 template <class T, class TT>
 constexpr size_t level_bytes() {
@@ -72,33 +105,18 @@ __global__ void __launch_bounds__(kThreads) k_implicit_columns_noalloc(int nz, i
     T* sb = sa + (size_t)wc * ld;
     T* sc = sb + (size_t)wc * ld;
     T* sd = sc + (size_t)wc * ld;
-    const T fact_tp = T(0.5) * (T(1.0) + beta);
-    const T fact_tm = T(0.5) * (T(1.0) - beta);
-    const T dt_tp2 = (dt * fact_tp) * (dt * fact_tp);
-    const T fact = fact_tm / fact_tp;
+    const Factors<T> f(grav, beta, dt);
     const size_t base = (size_t)j0 * nz;
     for (int e = threadIdx.x; e < nc * nz; e += kThreads) {
         const int col = e / nz, k = e - col * nz;
         if (k >= n) continue;
         const int o = col * ld + k;
-        const T* th = theta + base + e;    // this level of this column
-        const T* r2 = rt2pres + base + e;
-        const T* w = rho_w + base + e;
-        const T dz_k = grid.dz[k], dz_kp = grid.dz[k + 1], zd = grid.z[k + 1] - grid.z[k];
-        const T th_cur = moist::f2h(th[0], th[1], dz_k, dz_kp);
-        const T th_prev = k > 0 ? moist::f2h(th[-1], th[0], grid.dz[k - 1], dz_k) : T(0);
-        const T th_next = (k + 1 <= ke - 1) ? moist::f2h(th[1], th[2], dz_kp, grid.dz[k + 2]) : T(0);
-        const T b = dt_tp2 * (r2[0] / dz_k + r2[1] / dz_kp) * th_cur / zd;
-        const T a = (k > 0) ? -dt_tp2 * (r2[0] * th_prev / (zd * dz_k) - grav / (dz_k + dz_kp)) : T(0);
-        const T c = (k < ke - 1) ? -dt_tp2 * (r2[1] * th_next / (zd * dz_kp) + grav / (dz_k + dz_kp)) : T(0);
-        T d = w[0] + drho_w[base + e];
-        if (k > 0) d -= a * fact * w[0];
-        d -= b * fact * w[0];
-        if (k < ke - 1) d -= c * fact * w[1];
-        sa[o] = a;
-        sb[o] = b + T(1.0);
-        sc[o] = c;
-        sd[o] = d;
+        const size_t c0 = base + e;  // this level of this column
+        const Row<T> r = row_of(k, ke, f, grid, theta + c0, rt2pres + c0, rho_w + c0, drho_w + c0);
+        sa[o] = r.a;
+        sb[o] = r.b + T(1.0);
+        sc[o] = r.c;
+        sd[o] = r.d;
     }
     __syncthreads();
     if (threadIdx.x < nc) {
@@ -161,10 +179,66 @@ __global__ void __launch_bounds__(kThreads) k_implicit_columns_noalloc(int nz, i
     }
 }
 
+// Columns of few levels: one thread per column, everything in registers, IEEE division. A column is then a
+// sector or two of every array, and pieces of 8 columns leave most of a block's threads without a level: 262144
+// columns of 2 levels took 43.6 us, 65536 of 5 18.4 us, 29127 of 10 13.7 us that way (Float32, FP64 elimination),
+// 3.3, 4.5 and 7.3 us this way (5.1, 8.6 and 14.0 with one thread per column out of a scratch array). What bounds it
+// is the chain of quotients, so up to 64 columns an SM only the shortest columns take it: 6000 columns of
+// 5 levels 3.5 us against 3.9 in pieces, but 6000 of 8 5.0 against 4.6 (Float64 6.9 against 5.0).
+template <class T, class TT, int NZ>
+__global__ void __launch_bounds__(kThreads) k_implicit_columns_few(int ncols, T grav, T beta, T* rho_w,
+                                                                   const T* drho_w, const T* theta, const T* rt2pres,
+                                                                   T dt, const __grid_constant__ ColumnGrid<T, NZ> grid) {
+    constexpr int n = NZ - 1;
+    const int j = blockIdx.x * kThreads + threadIdx.x;
+    if (j >= ncols) return;
+    const Factors<T> f(grav, beta, dt);
+    const size_t base = (size_t)j * NZ;
+    TT cp[n], dp[n];
+#pragma unroll
+    for (int k = 0; k < n; k++) {
+        const size_t c0 = base + k;
+        const Row<T> r = row_of(k, NZ - 1, f, grid, theta + c0, rt2pres + c0, rho_w + c0, drho_w + c0);
+        const TT bb = (TT)(r.b + T(1.0));
+        if (k == 0) {
+            cp[0] = (TT)r.c / bb;
+            dp[0] = (TT)r.d / bb;
+        } else {
+            const TT piv = bb - (TT)r.a * cp[k - 1];
+            cp[k] = (TT)r.c / piv;
+            dp[k] = ((TT)r.d - (TT)r.a * dp[k - 1]) / piv;
+        }
+    }
+    TT x = dp[n - 1];
+    rho_w[base + n - 1] = (T)x;
+#pragma unroll
+    for (int k = n - 2; k >= 0; k--) {
+        x = dp[k] - cp[k] * x;
+        rho_w[base + k] = (T)x;
+    }
+}
+constexpr int FEW = 4, FEW_MANY = 10;  // levels: for any number of columns, for more than 64 an SM
+template <class T, class TT, int NZ = FEW_MANY>
+cudaError_t launch_few(const moist_params* p, int ncols, void* rho_w, const void* drho_w, const void* theta,
+                       const void* rt2pres, double dt, cudaStream_t st) {
+    if constexpr (NZ > 2) {
+        if (p->nz < NZ) return launch_few<T, TT, NZ - 1>(p, ncols, rho_w, drho_w, theta, rt2pres, dt, st);
+    }
+    ColumnGrid<T, NZ> grid;
+    std::memcpy(grid.dz, p->dz, sizeof grid.dz);
+    std::memcpy(grid.z, p->z, sizeof grid.z);
+    k_implicit_columns_few<T, TT, NZ><<<(ncols + kThreads - 1) / kThreads, kThreads, 0, st>>>(
+        ncols, (T)p->grav, (T)p->beta_offcenter, (T*)rho_w, (const T*)drho_w, (const T*)theta, (const T*)rt2pres,
+        (T)dt, grid);
+    return cudaGetLastError();
+}
+
 template <class T, class TT, int CAP>
 cudaError_t launch_noalloc(const moist_params* p, int ncols, void* rho_w, const void* drho_w, const void* theta,
                            const void* rt2pres, double dt, cudaStream_t st) {
     const int nz = p->nz;
+    if (nz <= FEW || (nz <= FEW_MANY && ncols > 64 * 148))
+        return launch_few<T, TT>(p, ncols, rho_w, drho_w, theta, rt2pres, dt, st);
     ColumnGrid<T, CAP> grid;  // levels from nz on are never read
     std::memcpy(grid.dz, p->dz, nz * sizeof(T));
     std::memcpy(grid.z, p->z, nz * sizeof(T));

@@ -109,6 +109,28 @@ def test_column_solve_strips(T, flags, nz, ncols, dt):
     assert np.array_equal(dev[0].cpu().numpy(), want)
 
 
+@pytest.mark.parametrize("nz,ncols", [(2, 1), (3, 131), (4, 9600), (5, 9472), (5, 9473), (7, 10001), (10, 9999), (11, 9999)])
+@pytest.mark.parametrize("T,flags", [(np.float32, 0), (np.float32, abi.MOIST_FLAG_TRI_NATIVE), (np.float64, 0)],
+                         ids=["f32-tri64", "f32-tri32", "f64"])
+def test_column_solve_of_few_levels(T, flags, nz, ncols):
+    """Both forms of the solve around the lines between them; 41 different columns, repeated."""
+    import torch
+    m = min(41, ncols)
+    p, arrays = _columns(T, nz, m, 6)
+    tri64 = T is np.float64 or not (flags & abi.MOIST_FLAG_TRI_NATIVE)
+    w, dw, th, r2 = [np.ascontiguousarray(np.resize(a, (ncols, nz))) for a in arrays]
+    want = arrays[0].copy()
+    for j in range(m):
+        col = want[j].copy()
+        bind.implicit_correction(col, dw[j].copy(), th[j].copy(), r2[j].copy(), T(0.25), p, tri64=tri64)
+        want[j] = col
+    dev = [torch.from_numpy(a).cuda() for a in (w, dw, th, r2)]
+    rc, msg = _call(p, flags, ncols, dev, T(0.25))
+    assert rc == abi.MOIST_OK, msg
+    torch.cuda.synchronize()
+    assert np.array_equal(dev[0].cpu().numpy(), np.resize(want, (ncols, nz)))
+
+
 @pytest.mark.parametrize("T,flags", [(np.float32, 0), (np.float32, abi.MOIST_FLAG_TRI_NATIVE), (np.float64, 0)],
                          ids=["f32-tri64", "f32-tri32", "f64"])
 @pytest.mark.parametrize("shapes", [[(6501, 9), (6397, 12), (6303, 7)],
