@@ -487,8 +487,9 @@ int moist_tracer_pass_counts(moist_ctx* ctx, int* counts, int n);
  * left and lower neighbours' new strips; every such wait gives up after `cycles` SM clock cycles
  * (cycles <= 0 restores the default, about two seconds), and the step then returns
  * MOIST_ERR_TIMEOUT, leaving the context's State undefined (upload a State before stepping
- * again). Meant for tests of that path. MOIST_ERR_UNSUPPORTED when the context's tracer sweep
- * does not wait (the streaming or wavefront sweep). */
+ * again). Meant for tests of that path. MOIST_ERR_UNSUPPORTED where the sweep has no limit to set:
+ * the wavefront sweep does not wait, and the waits of the streaming sweep's warps for their neighbours
+ * (also in ensembles: moist_batch_step) always end after about two seconds, with MOIST_ERR_TIMEOUT. */
 int moist_set_wait_limit(moist_ctx* ctx, long long cycles);
 
 /* Diagnostic of the tiled tracer sweep (no counterpart in the reference): runs nsteps large

@@ -148,6 +148,9 @@ cudaError_t device_info(DeviceInfo& out) {
     return cudaSuccess;
 }
 
+// the bound of a device-side wait: about two seconds
+inline long long wait_cycles(const DeviceInfo& d) { return (long long)d.clk_khz * 1000LL * 2; }
+
 inline unsigned cdiv(int a, int b) { return (unsigned)((a + b - 1) / b); }
 
 #define SINGLE_ARG(...) __VA_ARGS__
@@ -273,6 +276,7 @@ struct Ctx : CtxBase {
     // row-streaming tracer sweep (MOIST_FLAG_TRACER_STREAM)
     bool use_stream = false;
     T *skew_dom = nullptr, *skew_trc[3] = {nullptr, nullptr, nullptr};  // its records by anti-diagonal
+    long long stream_spin = 0;  // bound of its warps' waits, in SM clock cycles
     // column strips of the factorisation and the acoustic substeps
     int strip_wc = 1;
     size_t strip_smem = 0;
@@ -496,6 +500,7 @@ struct Ctx : CtxBase {
         for (int t = 0; t < 3; t++) AL(skew_trc[t], n * SK_NT);
         DeviceInfo di;
         CK(device_info(di));
+        stream_spin = wait_cycles(di);
         CK(cudaFuncSetAttribute(k_tracer_stream<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, di.optin));
         return MOIST_OK;
     }
@@ -565,7 +570,7 @@ struct Ctx : CtxBase {
         tctl.pass_ts = nullptr;
         tctl.pass_work = nullptr;
         tctl.timeout = err + 2;
-        tctl.spin_limit = (long long)di.clk_khz * 1000LL * 2;  // about two seconds
+        tctl.spin_limit = wait_cycles(di);
         wait_default = tctl.spin_limit;
         use_tiles = true;
         tiles_df = tiles_df_fit && (owner->flags & MOIST_FLAG_TRACER_DATAFLOW) != 0;
@@ -900,7 +905,7 @@ struct Ctx : CtxBase {
         tr.dt = dt_stage;
         MARK(MOIST_KGROUP_TRACER, use_stream || (use_tiles && tiles_df) ? 2 : 1);
         if (use_stream) {
-            StreamArgs<T> sa{tr, skew_dom, {skew_trc[0], skew_trc[1], skew_trc[2]}};
+            StreamArgs<T> sa{tr, skew_dom, {skew_trc[0], skew_trc[1], skew_trc[2]}, stream_spin};
             if (rec) {
                 rec->put(BK_PREP, BPrep<T>{dp, sa, err});
                 rec->put(BK_STREAM, BStream<T>{dp, sa, err});

@@ -43,6 +43,7 @@ struct StreamArgs {
     TracerArgs<T> tr;
     T* dom;      // [group][record][SK_ND][SK_ROWS]
     T* trc[3];   // [group][record][SK_NT][SK_ROWS]
+    long long spin_limit;  // bound of a wait for a neighbouring warp, in SM clock cycles
 };
 
 __device__ __forceinline__ int pmod(int c, int n) {
@@ -143,7 +144,6 @@ __host__ __device__ inline size_t stream_smem_bytes(int nz) {
     return (size_t)stream_groups(nz) * ((STREAM_RING * SK_REC + 2 * STREAM_TOP) * sizeof(T) + 2 * sizeof(int));
 }
 inline int stream_threads(int nz) { return stream_groups(nz) * 32; }
-constexpr long long STREAM_SPIN = 4000000000ll;  // bound of a wait for the neighbouring warp, in SM clock cycles (about 2 s)
 
 // one tracer t of one domain; blockDim.x = stream_threads(nz) or more. Returns (to every thread)
 // whether the fast division refused an operand or a result is not finite.
@@ -248,7 +248,7 @@ __device__ __forceinline__ bool stream_sweep(const DevParams<T>& p, const Stream
             if (lane == 0 && *count < least) {
                 const long long t0 = clock64();
                 while (*count < least)
-                    if (clock64() - t0 > STREAM_SPIN) {
+                    if (clock64() - t0 > a.spin_limit) {
                         ok = 0;
                         atomicExch(timeout, 1);
                         break;
