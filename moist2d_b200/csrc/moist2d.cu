@@ -589,7 +589,8 @@ struct Ctx : CtxBase {
             if (tctl.bar) CK(cudaMemsetAsync(tctl.bar, 0, 3 * sizeof(*tctl.bar), st));
             CK(reset_err());
             CK(cudaStreamSynchronize(st));
-            return set_err(owner, MOIST_ERR_TIMEOUT, "a bounded wait of the tracer sweep timed out");
+            return set_err(owner, MOIST_ERR_TIMEOUT, h[2] == 2 ? "the tiled tracer sweep did not converge within its bound of passes"
+                                                              : "a bounded wait of the tracer sweep timed out");
         }
         if (h[0] != INT_MAX) {
             owner->nan_field = h[0];

@@ -12,9 +12,11 @@
 // bottom neighbours' boundary strips (the stage-start values, which it forms itself), publishes
 // its own right and top strips whenever they change, and is recomputed only when a neighbour's
 // strip changed. A pass in which no strip changes leaves every tile computed from its neighbours'
-// final values: a fixed point, hence the reference's result bit for bit. Influence between cells
-// decays roughly like the Courant number per cell, so two or three passes suffice; the pass count
-// is bounded by tiles_x + tiles_z + 1 (information crosses one tile per pass).
+// final values: a fixed point, hence the reference's result bit for bit. Information crosses one
+// tile per pass, so a chunk needs at most its tile columns + tiles_z passes; max_pass leaves two to
+// spare, and a sweep that reached it would report an error, never a result. Mostly a few passes
+// do, but a change of one ulp can keep reproducing itself along uniform rows: on spun-up States 3-4 on
+// 200 x 100 in Float32 and 5-8 in Float64, 11-16 on 2048 x 128 in Float64, 12-33 on 4096 x 256.
 //
 // The kernel is persistent (cooperative launch, the tiles of a chunk resident); passes are
 // separated by a grid barrier whose wait is bounded: on timeout it records MOIST_ERR_TIMEOUT and
@@ -47,7 +49,7 @@ struct TileCtl {
     int* changed;       // [2][3][ntiles][2] per pass parity: rows whose right-strip entries changed, columns whose top-strip entries changed (bit masks)
     int* passes;        // out: passes run (all chunks)
     int* hist;          // [64] sweeps that converged after p passes
-    int* timeout;       // out: barrier timeout flag
+    int* timeout;       // out: 1: a wait ran out, 2: no fixed point within max_pass
     long long spin_limit;
     unsigned long long* pass_ts;  // optional diagnostic [max_pass + 3] of the first chunk: globaltimer at the
                                   // start of each pass, and at [max_pass + 2] when block 0 leaves it
@@ -446,7 +448,10 @@ __global__ void __launch_bounds__(96, sizeof(T) == 4 ? 4 : 2) k_tracer_tiles(Dev
         int pass = 1;
         for (;; pass++) {
             if constexpr (!DF) {
-                if (pass > ctl.max_pass) break;
+                if (pass > ctl.max_pass) {  // changes still under way: the bound does not hold (all blocks alike)
+                    if (threadIdx.x == 0) atomicMax(ctl.timeout, 2);
+                    return;
+                }
             }
             const int cur = pass & 1, prv = cur ^ 1;
             unsigned lmask = 0u, bmask = 0u;

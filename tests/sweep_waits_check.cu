@@ -3,6 +3,8 @@
 //   stream nx nz limit   the streaming sweep (k_stream_prep, k_tracer_stream) with waits of at most `limit`
 //                        cycles: "<timeout word> <mismatches>", the results against those of the
 //                        wavefront sweep (k_tracer_wavefront, IEEE division)
+//   tiles nx nz passes   the tiled sweep (k_tracer_tiles, one chunk) with a bound of `passes` passes: likewise
+//
 // The domain has cloud-like tracers, both signs of wind, a stretched grid.
 #include <climits>
 #include <cstdio>
@@ -89,6 +91,26 @@ int main(int argc, char** argv) {
         cudaFuncSetAttribute(k_tracer_stream<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         k_stream_prep<T><<<dim3((nx + 34) / 32, (nz + 31) / 32), 256>>>(p, s, err);
         k_tracer_stream<T><<<3, stream_threads(nz), smem>>>(p, s, err);
+    } else if (!strcmp(argv[1], "tiles")) {
+        TileCtl c{};
+        c.tiles_x = c.chunk_x = (nx + TT_W - 1) / TT_W;
+        c.tiles_z = (nz + TT_H - 1) / TT_H;
+        c.ntiles = c.tiles_x * c.tiles_z;
+        c.max_pass = (int)limit;
+        c.bar = device(std::vector<unsigned long long>(3));
+        c.changed = device(std::vector<int>((size_t)2 * 3 * c.ntiles * 2));
+        c.passes = device(std::vector<int>(1));
+        c.hist = device(std::vector<int>(64));
+        c.timeout = err + 2;
+        c.spin_limit = 4000000000ll;
+        T* strips = device(std::vector<T>((size_t)TT_RING * 3 * c.ntiles * 4 * TT_W));
+        const int smem = (int)sizeof(TileSmem<T>);
+        cudaFuncSetAttribute(k_tracer_tiles<T, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+        const int* e = err;
+        void* args[] = {&p, &a, &c, &strips, &e};
+        if (cudaLaunchCooperativeKernel((void*)k_tracer_tiles<T, false>, dim3(c.ntiles), dim3(96), args, smem, 0) !=
+            cudaSuccess)
+            return 2;
     } else {
         return 2;
     }

@@ -280,6 +280,19 @@ def test_adjoint_tiny_shapes_forward_mode(nx, nz):
     tangent_check(p, s, 3, prec_w, seeds, g, ndir=3, seed=nx * 10 + nz)
 
 
+@pytest.mark.parametrize("nx,nz", [(4, 7), (33, 45), (5, 517)])
+def test_adjoint_reverse_sweep_records_forward_mode(nx, nz):
+    """Odd row counts (the reverse tracer sweep's records are padded), more than 512 rows (its ring holds four
+    records instead of eight), and four columns, where the gathers' neighbours two to the left and right coincide."""
+    from states import small_case
+    grid = dict(dz0=20.0, H=20.0 * nz * 1.02) if nz > 250 else {}
+    p, s = small_case(np.float64, nx, nz, do_sf=False, do_rd=False, **grid)
+    prec_w = rain_weight(p)
+    seeds = state_seeds(p, s, 17)
+    g, _ = run_adjoint(p, s, 3, 2, prec_w, seeds)
+    tangent_check(p, s, 3, prec_w, seeds, g, ndir=3, seed=nx + nz)
+
+
 FIXTURE_RTOL = 1e-12
 
 

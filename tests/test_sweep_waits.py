@@ -2,7 +2,8 @@
 the tiled sweep's (test_wait_limit.py); the warps of the streaming sweep, which ensembles always run, wait
 for their neighbours within a limit that the launch carries. One cycle makes these waits run out: the sweep
 then ends by itself and sets the timeout word. With the default's two seconds it never does, and the
-results are those of the wavefront sweep bit for bit."""
+results are those of the wavefront sweep bit for bit. Likewise the tiled sweep's bound of passes: a sweep
+that reaches it before its fixed point ends with the error word set."""
 import os
 import subprocess
 
@@ -32,3 +33,10 @@ def test_stream_waits(checker, nx, nz):
     timeout, _ = run(checker, "stream", nx, nz, 1)
     assert timeout == 1
     assert run(checker, "stream", nx, nz, LONG) == [0, 0]
+
+
+@pytest.mark.parametrize("nx,nz", [(70, 17), (300, 48), (129, 250)])
+def test_tiles_pass_bound(checker, nx, nz):
+    error, mismatches = run(checker, "tiles", nx, nz, 1)
+    assert error == 2 and mismatches > 0
+    assert run(checker, "tiles", nx, nz, -(-nx // 32) + -(-nz // 16) + 2) == [0, 0]

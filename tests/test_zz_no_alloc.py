@@ -90,3 +90,31 @@ def test_noalloc_refuses_sizes_beyond_its_limits():
     assert rc == abi.MOIST_ERR_ARG and b"limit" in msg
     torch.cuda.synchronize()
     assert torch.equal(buf, before)  # nothing was queued
+
+
+@pytest.mark.parametrize("T,flags", MODES, ids=["f32-tri64", "f32-tri32", "f64"])
+def test_noalloc_calls_on_two_streams_are_independent(T, flags):
+    """Different systems queued on two streams, with nothing between them that waits, and again for several rounds:
+    every call gives what it gives alone."""
+    import torch
+    jobs = []
+    for j, (nz, ncols) in enumerate([(97, 900), (64, 1200), (5, 9600)]):
+        p, arrays = _columns(T, nz, ncols, 40 + j)
+        dev = [torch.from_numpy(a).cuda() for a in arrays]
+        alone = [dev[0].clone()] + dev[1:]
+        rc, msg = _call(p, flags, ncols, alone, T(0.25))
+        assert rc == abi.MOIST_OK, msg
+        jobs.append((p, ncols, dev, alone[0]))
+    torch.cuda.synchronize()
+    streams = [torch.cuda.Stream() for _ in range(2)]
+    outs = []
+    for rep in range(6):
+        for j, (p, ncols, dev, want) in enumerate(jobs):
+            with torch.cuda.stream(streams[(rep + j) % 2]):
+                bufs = [dev[0].clone()] + dev[1:]
+                rc, msg = _call(p, flags, ncols, bufs, T(0.25))
+                assert rc == abi.MOIST_OK, msg
+            outs.append((bufs[0], want))
+    torch.cuda.synchronize()
+    for got, want in outs:
+        assert torch.equal(got, want)
