@@ -1265,6 +1265,12 @@ __host__ __device__ inline size_t strip_smem_bytes(int nz, int wc) {
     return 8 * n * sizeof(TT) + (2 * (size_t)nz * wc + (size_t)nz * (wc + 1)) * sizeof(T);
 }
 
+// The most that a strip may take for two blocks to share an SM (228 KB, of which each block takes one more):
+// 8 columns of up to 184 levels in Float32 with the FP64 elimination, of up to 157 in Float64. Past it one block runs at
+// a time and half the columns are faster: 1300 x 187 in Float32 1.45 ms a step with 4 columns, 1.59 with 8,
+// in Float64 1300 x 160 3.66 and 3.80; below it 8 are: 1300 x 180 1.33 against 1.41 with 4.
+constexpr size_t STRIP_SMEM_TWO = 112 * 1024;
+
 // A loop whose iterations load from global memory and then compute, in batches: every thread
 // loads the operands of SUB_BATCH iterations (load(e) returns them) before computing any
 // (work(e, v)), so that it waits for one memory round trip per batch instead of one per

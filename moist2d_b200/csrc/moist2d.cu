@@ -518,7 +518,7 @@ struct Ctx : CtxBase {
         const int nsm = di.nsm, optin = di.optin;
         strip_wc = 1;
         for (int w : {8, 4, 2}) {
-            if (cdiv(nx, w) >= nsm && strip_smem_bytes<T, TT>(nz, w) <= 96 * 1024) {
+            if (cdiv(nx, w) >= nsm && strip_smem_bytes<T, TT>(nz, w) <= STRIP_SMEM_TWO) {
                 strip_wc = w;
                 break;
             }
@@ -2590,13 +2590,20 @@ struct BatchImpl : BatchBase {
 
     int build() {
         const int n = (int)m.size();
+        DeviceInfo di;
+        BCK(device_info(di));
+        long cols = 0;
+        for (auto* c : m) cols += c->nx;
         for (auto* c : m) {
             cur0.push_back(c->cur);
             nxt0.push_back(c->nxt);
-            // a batch has blocks enough for every SM without narrow strips: take the widest
-            // strip whose shared memory leaves room for several blocks per SM
+            // The widest strip of which two fit on an SM, as many as the kernels' registers allow (16 members of
+            // 512 and 1024 columns, strips bounded to 64 KB: 4 columns of 128 levels 6.35 ms a step, 8 5.48; of 256
+            // levels 2 14.5, 4 10.9; Float64 13.9 and 13.0, 24.3 and 20.2); fewer columns where the whole batch would
+            // have strips for less than two thirds of the SMs (512 columns of 128 levels: 8 2.01 ms, 4 1.96; 600
+            // of 100 in Float64 2.48 and 2.43).
             for (int w : {8, 4, 2, 1}) {
-                if (w == 1 || strip_smem_bytes<T, TT>(c->nz, w) <= 64 * 1024) {
+                if (w == 1 || (strip_smem_bytes<T, TT>(c->nz, w) <= STRIP_SMEM_TWO && cols / w >= 2 * di.nsm / 3)) {
                     c->strip_wc = w;
                     c->strip_smem = strip_smem_bytes<T, TT>(c->nz, w);
                     break;
@@ -2658,14 +2665,14 @@ struct BatchImpl : BatchBase {
         }
         BCK(cudaEventCreateWithFlags(&gfork, cudaEventDisableTiming));
         // The forms before any autotuning. Up to 128 columns per SM the factorisation and substep run over
-        // column strips: one thread per column leaves the SMs waiting for its chain (6 members, 4600
-        // columns: 6.8 ms a step per column, 4.0 over strips); beyond, one thread per column wins (64 members,
-        // 74000 columns: 24.4 over strips, 16.8 per column), in Float32 best in blocks of 128 with the
-        // registers of three blocks of 256 (form 3; form 4 in blocks of 64: 17.6).
-        DeviceInfo di;
-        BCK(device_info(di));
-        long cols = 0;
-        for (auto* c : m) cols += c->nx;
+        // column strips: one thread per column leaves the SMs waiting for its chain. Ms a step of members of
+        // 512 and 1024 columns, strips / per column, Float32: of 96 and 128 levels 3.4 / 7.0 at 3000 columns, 5.4 / 8.2 at
+        // 12800, 6.7 / 8.6 at 19000, 8.0 / 9.5 at 25000, 9.6 / 10.1 at 32000, 12.3 / 11.6 at 44000; of 64 levels 4.8 / 5.5 at
+        // 18000, 5.7 / 6.0 at 25000, 6.6 / 6.4 at 31000; of 256 10.9 / 14.8 at 11000, 15.4 / 16.0 at 18000, 19.4 / 17.5 at
+        // 25000. In Float64 the two meet at 18000 (256 levels) to 35000 columns. The line is where the tallest
+        // members' forms meet, the only ones that lose much on its far side. Beyond it one thread per column, in Float32 in
+        // blocks of 128 with the registers of three blocks of 256 (form 3: 64 members 16.8 ms, form 4 in
+        // blocks of 64 17.6; at 25000 to 44000 columns form 4 is 3 to 4 % faster than form 3).
         sub_strips = cols <= 128L * di.nsm;
         if (!sub_strips && sizeof(T) == 4) {
             sub_form = 3;

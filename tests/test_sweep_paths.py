@@ -145,3 +145,21 @@ def test_ensembles_of_many_columns(T, flags, shapes):
         got = [e.download(i, s.copy()) for i, (_, s) in enumerate(mem)]
     for (p, s), g in zip(mem, got):
         compare(g, model.rk3_step(s.copy(), p, 3, flags=flags), p)
+
+
+@pytest.mark.parametrize("T,flags,nzs", [(np.float32, 0, (184, 185)), (np.float32, abi.MOIST_FLAG_TRI_NATIVE, (256, 129)),
+                                         (np.float64, 0, (157, 158))], ids=["f32-tri64", "f32-tri32", "f64"])
+@pytest.mark.parametrize("nx", [395, 150, 50])
+def test_ensemble_strips_at_the_most_shared_memory(T, flags, nzs, nx):
+    """Column strips of the widest width, the last level count that has it and the first that has not, with
+    columns enough for it and for half and a quarter of it."""
+    mem = [small_case(T, nx, nz, dz0=50.0, H=50.0 * nz * 1.02) for nz in nzs]
+    with model.Ensemble([p for p, _ in mem], flags) as e:
+        for i, (_, s) in enumerate(mem):
+            e.upload(i, s)
+        e.step(2)
+        got = [e.download(i, s.copy()) for i, (_, s) in enumerate(mem)]
+    for (p, s), g in zip(mem, got):
+        o = s.copy()
+        bind.rk3_step(o, p, 2, tri64=not flags)
+        compare(g, o, p)
