@@ -234,7 +234,8 @@ int moist_implicit_correction(const moist_params* p, int precision, int flags, v
  * Limits: nz <= MOIST_NOALLOC_MAX_NZ, and 2*(nz-1)*ncols*sizeof(elimination type) <=
  * MOIST_NOALLOC_SCRATCH_BYTES (e.g. 2048 columns of 128 levels with the FP64 elimination);
  * larger calls return MOIST_ERR_ARG before queuing anything and write the reason to err (if not
- * NULL). Calls on different streams and from different threads are independent of one another. */
+ * NULL). The second limit is the call's contract, from when that scratch was an array in device memory;
+ * none is allocated now. Calls on different streams and from different threads are independent of one another. */
 #define MOIST_NOALLOC_MAX_NZ 1024
 #define MOIST_NOALLOC_SCRATCH_BYTES (4 * 1024 * 1024)
 int moist_implicit_correction_noalloc(const moist_params* p, int precision, int flags, int ncols,

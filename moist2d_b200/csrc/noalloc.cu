@@ -262,8 +262,8 @@ int run_noalloc(const moist_params* p, int ncols, void* rho_w, const void* drho_
     if (work_bytes > MOIST_NOALLOC_SCRATCH_BYTES) {
         char msg[256];
         std::snprintf(msg, sizeof msg,
-                      "moist_implicit_correction_noalloc: %d columns of %d levels need %zu scratch bytes, "
-                      "more than the fixed %d-byte scratch array",
+                      "moist_implicit_correction_noalloc: %d columns of %d levels are %zu scratch bytes of elimination, "
+                      "more than the %d that a call takes (MOIST_NOALLOC_SCRATCH_BYTES)",
                       ncols, nz, work_bytes, (int)MOIST_NOALLOC_SCRATCH_BYTES);
         put_msg(err, errlen, msg);
         return MOIST_ERR_ARG;

@@ -118,3 +118,12 @@ def test_noalloc_calls_on_two_streams_are_independent(T, flags):
     torch.cuda.synchronize()
     for got, want in outs:
         assert torch.equal(got, want)
+
+
+def test_noalloc_refusal_names_the_limit_and_no_array():
+    import torch
+    buf = torch.zeros(16, dtype=torch.float32, device="cuda")
+    p = Params(np.float32, Nx=2, Nz=128, H=100.0 * 128 * 1.02, dz0=100.0, z_fact=1.05)
+    rc, msg = _call(p, 0, 5000, [buf] * 4, 0.1)
+    assert rc == abi.MOIST_ERR_ARG
+    assert b"MOIST_NOALLOC_SCRATCH_BYTES" in msg and b"4194304" in msg and b"array" not in msg
