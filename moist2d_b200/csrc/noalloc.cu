@@ -237,7 +237,11 @@ template <class T, class TT, int CAP>
 cudaError_t launch_noalloc(const moist_params* p, int ncols, void* rho_w, const void* drho_w, const void* theta,
                            const void* rt2pres, double dt, cudaStream_t st) {
     const int nz = p->nz;
-    if (nz <= FEW || (nz <= FEW_MANY && ncols > 64 * 148))
+    int dev = 0, nsm = 0;
+    cudaError_t e = cudaGetDevice(&dev);
+    if (e == cudaSuccess) e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+    if (e != cudaSuccess) return e;
+    if (nz <= FEW || (nz <= FEW_MANY && ncols > 64 * nsm))
         return launch_few<T, TT>(p, ncols, rho_w, drho_w, theta, rt2pres, dt, st);
     ColumnGrid<T, CAP> grid;  // levels from nz on are never read
     std::memcpy(grid.dz, p->dz, nz * sizeof(T));
@@ -246,7 +250,7 @@ cudaError_t launch_noalloc(const moist_params* p, int ncols, void* rho_w, const 
     // levels takes 48 KiB in Float64) or while the blocks are fewer than the SMs, whose chains run side by side
     auto bytes = [&](int w) { return level_bytes<T, TT>() * column_stride(nz, w) * w; };
     int wc = 8;
-    while (wc > 1 && (bytes(wc) > 48 * 1024 || (ncols + wc - 1) / wc < 148)) wc /= 2;
+    while (wc > 1 && (bytes(wc) > 48 * 1024 || (ncols + wc - 1) / wc < nsm)) wc /= 2;
     k_implicit_columns_noalloc<T, TT, CAP><<<(ncols + wc - 1) / wc, kThreads, bytes(wc), st>>>(
         nz, ncols, wc, (T)p->grav, (T)p->beta_offcenter, (T*)rho_w, (const T*)drho_w, (const T*)theta,
         (const T*)rt2pres, (T)dt, grid);
