@@ -3,16 +3,15 @@
 // CUDA's IEEE division ends every quotient with a range check and a branch to a slow path (very
 // slow for subnormal results), so consecutive divisions cannot overlap and the code between them
 // cannot be scheduled together: a tracer cell of ~25 such divisions is ~1800 cycles of dependent
-// latency, and the Gauss-Seidel tracer sweep walks long chains of cells. Three policies:
+// latency, and the Gauss-Seidel tracer sweep walks long chains of cells. In its place:
 //   FastDiv<T> (tracer cell, column solve): remainder corrections in the type's own precision; what
 //       it cannot round exactly is reported and the caller repeats with IeeeDiv<T>;
-//   RN32(RN64(a y)) with y = 1/b in double precision (div64; slow tendencies), the IEEE quotient of
-//       floats but for ties in the subnormal range, which a guard word reports (Div64) or explicit
-//       rounding resolves (Div64X);
-//   qdiv_checked / quotient_proven (Thomas recurrences): a corrected double quotient with an exact
-//       acceptance test.
-// tests/fastdiv_check.cu and tests/celldiv_check.cu compare them with IEEE division on the GPU, over
-// all numerators for the model's denominators and on random bit patterns of every class.
+//   div64 (slow tendencies): RN32(RN64(a y)) with a tabulated y = 1/b in double precision, the IEEE
+//       quotient of floats but for ties in the subnormal range, which a guard word reports;
+//   quotient_proven (acoustic substep): an exact test of a corrected double quotient, beside the
+//       recurrence.
+// tests/fastdiv_check.cu, tests/celldiv_check.cu and tests/quotient_check.cu compare them with IEEE division on
+// the GPU, over all numerators for the model's denominators and on random bit patterns of every class.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -27,22 +26,8 @@ __device__ __forceinline__ float with_sign_of(float q, float q0) {
     return __int_as_float(__float_as_int(q) | (__float_as_int(q0) & (int)0x80000000));
 }
 
-// Selects the compiler cannot turn into branches: both operands are always computed, so the
+// A select the compiler cannot turn into a branch: both operands are always computed, so the
 // independent parts of a cell update stay in one basic block and overlap.
-__device__ __forceinline__ float sel_gt(float a, float b, float x, float y) {  // a > b ? x : y
-    float r;
-    asm("{\n\t.reg .pred p;\n\tsetp.gt.f32 p, %1, %2;\n\tselp.f32 %0, %3, %4, p;\n\t}"
-        : "=f"(r) : "f"(a), "f"(b), "f"(x), "f"(y));
-    return r;
-}
-__device__ __forceinline__ float sel_lt(float a, float b, float x, float y) {  // a < b ? x : y
-    float r;
-    asm("{\n\t.reg .pred p;\n\tsetp.lt.f32 p, %1, %2;\n\tselp.f32 %0, %3, %4, p;\n\t}"
-        : "=f"(r) : "f"(a), "f"(b), "f"(x), "f"(y));
-    return r;
-}
-__device__ __forceinline__ double sel_gt(double a, double b, double x, double y) { return a > b ? x : y; }
-__device__ __forceinline__ double sel_lt(double a, double b, double x, double y) { return a < b ? x : y; }
 __device__ __forceinline__ double sel_u(unsigned c, double x, double y) { return c != 0 ? x : y; }
 __device__ __forceinline__ float sel_u(unsigned c, float x, float y) {  // c != 0 ? x : y
     float r;
@@ -123,8 +108,10 @@ __device__ __forceinline__ double rcp64(float b) {
     return __fma_rn(y, e, y);
 }
 
-// division policies by the double reciprocal: cdiv(a, b, y, g) with y = 1/b prepared once,
-// vdiv(a, b, g) for a variable denominator, div3(a) = a / 3; g is the subnormal guard word
+// Division by the double reciprocal: cdiv(a, b, y, g) with y = 1/b prepared once is what the slow
+// tendencies do (div64 and the guard); the variable denominator (vdiv, rcp64) and the explicit rounding
+// (Div64X, div64x) are compared with IEEE division by tests/fastdiv_check.cu and not used by any
+// kernel. g is the subnormal guard word.
 struct Div64 {  // FP64 reciprocal: exact for every input but subnormal ties, which g reports
     using R = double;
     __device__ __forceinline__ static R rcp(float b) { return 1.0 / (double)b; }
@@ -138,15 +125,12 @@ struct Div64 {  // FP64 reciprocal: exact for every input but subnormal ties, wh
         subnormal_guard(g, q);
         return q;
     }
-    // (1 + 2r) / 3: the numerator is 0 or at least 2^-24 in magnitude, so no subnormal quotient
-    __device__ __forceinline__ static float div3(float a) { return div64(a, 1.0 / 3.0); }
 };
 struct Div64X {  // FP64 reciprocal with explicit rounding of subnormal quotients: exact for every input
     using R = double;
     __device__ __forceinline__ static R rcp(float b) { return 1.0 / (double)b; }
     __device__ __forceinline__ static float cdiv(float a, float, R y, unsigned&) { return div64x(a, y); }
     __device__ __forceinline__ static float vdiv(float a, float b, unsigned&) { return div64x(a, rcp64(b)); }
-    __device__ __forceinline__ static float div3(float a) { return div64(a, 1.0 / 3.0); }
 };
 
 // ---- division in the type's own arithmetic: remainder corrections on a reciprocal
@@ -291,23 +275,18 @@ struct IeeeDiv {
     __device__ __forceinline__ static T div6(T a) { return a / T(6); }
 };
 
-// ---- the correctly rounded double quotient a/b without a division on the dependent path
+// ---- exact test of a double quotient
 //
-// Given y = RN(1/b) (formed ahead, off the path): q0 = RN(a y) lies within 1.5 ulp of a/b; one
-// correction with its remainder, q1 = RN(q0 + (a - b q0) y), brings it to the correctly rounded
-// quotient in all but rare cases. q1 is then checked exactly: when q1 lies within one ulp of
-// a/b, the remainder r1 = a - b q1 is a double and the FMA forms it exactly (no underflow for
-// the operand ranges admitted below), and |r1| < |b| u/2, with u the smaller of the two ulps
-// around q1 (the ulp below a power of two is half the one above), says that a/b is nearer to
-// q1 than to the midpoint towards either neighbour, i.e. q1 = RN(a/b). |b| u/2 is a power-of-two
-// multiple of b, hence exact. When q1 is farther than one ulp the computed |r1| is at least
-// RN(|b| u) = 2 (|b| u/2), so the test fails. ok is cleared where the test fails or the operands
-// leave 2^-960 <= |a| <= 2^1000, 2^-1000 <= |b| <= 2^1000 (non-finite values included): the
-// caller then divides again with IEEE division. a = 0 gives q0 = a y, the IEEE result with its
-// sign. The method is the remainder correction of Markstein's division (IBM J. Res. Dev. 34,
-// 1990) with an exact acceptance test in place of a proof for every operand. On B200 the
-// dependent path is 69 cycles against 112 for IEEE division (with the multiply-subtract of a
-// Thomas level in both).
+// Let q1 be near a/b: the acoustic substep forms it from y = RN(1/b) with one correction by the
+// remainder, q1 = RN(q0 + (a - b q0) y), which is the correctly rounded quotient in all but rare cases
+// (Markstein, IBM J. Res. Dev. 34, 1990). When q1 lies within one ulp of a/b, the remainder
+// r1 = a - b q1 is a double and the FMA forms it exactly (no underflow for the operand ranges admitted
+// below), and |r1| < |b| u/2, with u the smaller of the two ulps around q1 (the ulp below a power of
+// two is half the one above), says that a/b is nearer to q1 than to the midpoint towards either
+// neighbour, i.e. q1 = RN(a/b). |b| u/2 is a power-of-two multiple of b, hence exact. When q1 is farther
+// than one ulp the computed |r1| is at least RN(|b| u) = 2 (|b| u/2), so the test fails. It also fails
+// where the operands leave 2^-960 <= |a| <= 2^1000, 2^-1000 <= |b| <= 2^1000 (non-finite values
+// included): the caller then divides again with IEEE division.
 __device__ __forceinline__ bool quotient_proven(double a, double b, double q1) {
     const double r1 = fma(-b, q1, a);
     const unsigned long long bits = (unsigned long long)__double_as_longlong(q1) & 0x7fffffffffffffffULL;
@@ -317,14 +296,6 @@ __device__ __forceinline__ bool quotient_proven(double a, double b, double q1) {
     const double aa = fabs(a), ab = fabs(b);
     const bool in_range = aa >= 0x1p-960 && aa <= 0x1p1000 && ab >= 0x1p-1000 && ab <= 0x1p1000 && he >= 1;
     return in_range && fabs(r1) < ab * half_u;
-}
-__device__ __forceinline__ double qdiv_checked(double a, double b, double y, bool& ok) {
-    const double q0 = a * y;
-    const double r0 = fma(-b, q0, a);
-    const double q1 = fma(r0, y, q0);
-    const bool zero = a == 0.0;
-    ok = ok && (zero || quotient_proven(a, b, q1));
-    return zero ? q0 : q1;
 }
 
 }  // namespace moist
