@@ -79,12 +79,13 @@ enum {
     /* Run the tracer transport as one exact wavefront per tracer instead of the tiled sweep
      * (same results bit for bit, much slower; kept for cross-checking). */
     MOIST_FLAG_TRACER_WAVEFRONT = 2,
-    /* Run the tracer transport as one exact row-streaming wavefront per tracer (one thread per
-     * row; no repair passes; same results bit for bit). Needs nz <= 256. */
+    /* Run the tracer transport as one exact row-streaming wavefront per tracer (a warp per 16 rows,
+     * two lanes per cell; no repair passes; same results bit for bit). Needs nz <= 256. */
     MOIST_FLAG_TRACER_STREAM = 4,
     /* Run the tiled tracer sweep without grid-wide passes: each tile publishes numbered versions
      * of its boundary strips and recomputes as soon as its left or lower neighbour publishes a
-     * new one (same results bit for bit). */
+     * new one (same results bit for bit). Every tile has to be resident on the GPU: a domain whose
+     * tiles are not runs the sweep with passes, in chunks of tile columns. */
     MOIST_FLAG_TRACER_DATAFLOW = 8
 };
 

@@ -92,8 +92,8 @@ __device__ __forceinline__ T tanh_m(T x) {  // tanh from the shared exp
 // once for all cells in parallel, the two flux recurrences (up on one thread per column, down on
 // another) run out of shared memory, the heating rates over all cells again. One thread per column
 // formed every cell's powers three times in the order of the recurrences: 1.38 ms for 640 x 250
-// (Float32; 20 warps on the GPU), 0.04 ms this way. wc: 8, or fewer where 148 blocks or the shared
-// memory of two blocks per SM ask for it (rd_strip).
+// (Float32; 20 warps on the GPU), 0.04 ms this way. wc: 8, or fewer where a block for every SM or the
+// shared memory of two blocks per SM asks for it (rd_strip).
 constexpr int RD_THREADS = 256;
 template <class T>
 __host__ __device__ inline size_t rd_smem_bytes(int nz, int wc) {
