@@ -448,10 +448,7 @@ __global__ void __launch_bounds__(96, sizeof(T) == 4 ? 4 : 2) k_tracer_tiles(Dev
         int pass = 1;
         for (;; pass++) {
             if constexpr (!DF) {
-                if (pass > ctl.max_pass) {  // changes still under way: the bound does not hold (all blocks alike)
-                    if (threadIdx.x == 0) atomicMax(ctl.timeout, 2);
-                    return;
-                }
+                if (pass > ctl.max_pass) break;
             }
             const int cur = pass & 1, prv = cur ^ 1;
             unsigned lmask = 0u, bmask = 0u;
@@ -638,6 +635,7 @@ __global__ void __launch_bounds__(96, sizeof(T) == 4 ? 4 : 2) k_tracer_tiles(Dev
             }
         } else if (blockIdx.x == 0 && threadIdx.x == 0) {
             if (ctl.pass_ts && tx0 == 0) ctl.pass_ts[ctl.max_pass + 2] = globaltimer_ns();  // block 0 leaves the chunk
+            if (pass > ctl.max_pass) atomicMax(ctl.timeout, 2);  // no fixed point: what was written is no result
         }
         __syncthreads();  // the next chunk stages over this one's shared memory
     }
