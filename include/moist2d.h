@@ -231,7 +231,7 @@ int moist_implicit_correction(const moist_params* p, int precision, int flags, v
  * starts at element j*nz); p->dz, p->z (host) give the grid and travel in the kernel's
  * parameter block; p->grav and p->beta_offcenter are read. The work is queued on `stream` (a
  * cudaStream_t, NULL = default stream) and the call returns without waiting; it issues no
- * memory copy. It calls no cudaMalloc or cudaFree: the elimination works in shared memory.
+ * memory copy. It calls no cudaMalloc or cudaFree: the elimination works in shared memory and registers.
  * Limits: nz <= MOIST_NOALLOC_MAX_NZ, and 2*(nz-1)*ncols*sizeof(elimination type) <=
  * MOIST_NOALLOC_SCRATCH_BYTES (e.g. 2048 columns of 128 levels with the FP64 elimination);
  * larger calls return MOIST_ERR_ARG before queuing anything and write the reason to err (if not

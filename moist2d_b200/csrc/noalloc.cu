@@ -8,7 +8,7 @@
 // keeps other streams busy cannot afford cudaFree, which waits for the whole device.
 // moist_implicit_correction allocates its column buffers on every call; this variant
 // allocates nothing. The grid vectors travel in the kernel's parameter block (so the call
-// issues no host-to-device copy either), and the elimination works in shared memory.
+// issues no host-to-device copy either), and the elimination works in shared memory and registers.
 #include <cuda_runtime.h>
 
 #include <cstdio>
